@@ -21,12 +21,12 @@ cudaError_t launch_nsol(int prec, int lay, const StepParams &p, unsigned t, dim3
             return cudaGetLastError();
         }
         switch (prec * 3 + lay) {
-            PLBM_ALL_CASES(k_nsol_even)
+            PLBM_ALL_CASES_2(k_nsol_even_bound, k_nsol_even)
         default: return cudaErrorInvalidValue;
         }
     } else {
         switch (prec * 3 + lay) {
-            PLBM_ALL_CASES(k_nsol_odd)
+            PLBM_ALL_CASES_2(k_nsol_odd_bound, k_nsol_odd)
         default: return cudaErrorInvalidValue;
         }
     }

@@ -26,6 +26,7 @@
 #include <stdint.h>
 
 #include "plbm_params.h"
+#include "plbm_strict.cuh"
 
 namespace plbm {
 
@@ -149,6 +150,9 @@ struct Moments { double rho, jx, jy, usq; };
 // The float forms keep their moments in float: GB300 issues FP64 at 1/64 of the FP32 rate, so
 // they are widened to double only on the steps that write them (observables<PREC>).
 struct MomentsF { float rho, jx, jy, usq; };
+// F64_STRICT: rho, jx, jy as fixed point (x * 2^61) and u^2 * 2^122 when `fixed`, otherwise the bits
+// of the doubles; converted where they are written (observables<F64_STRICT>).
+struct MomentsS { long long rho, jx, jy; double usq; bool fixed; };
 
 __device__ __forceinline__ double nan_guard(double v)
 {
@@ -159,7 +163,9 @@ __device__ __forceinline__ double nan_guard(double v)
 // F64_STRICT: the reference's StreamCollideKernel arithmetic (nptl_kernels.hpp:382-409) in its
 // exact IEEE operation order, every operation rounded separately (no contraction).  Terms the
 // reference multiplies by a velocity component of 0 or +-1 are exact and are written as the
-// sums and negations they reduce to; the results are the same values.
+// sums and negations they reduce to; the results are the same values.  This is the form for
+// populations outside the range of strict::fast_collide; it is bound by the FP64 pipe (97
+// instructions a node at about two lanes per cycle and SM).
 __device__ __forceinline__ Moments collide_f64_strict(double f[9], double omega)
 {
     double rho = f[0];
@@ -417,13 +423,35 @@ __device__ __forceinline__ Moments collide_q60(long long f[9], const StepParams 
     return { __longlong_as_double(rho), __longlong_as_double(jx), __longlong_as_double(jy), __longlong_as_double(usq) };
 }
 
+// F64_STRICT on the integer pipe where the node's values allow it (strict::fast_collide: the same
+// doubles), on the FP64 pipe otherwise.
+__device__ __forceinline__ MomentsS collide_strict(double f[9], double omega)
+{
+    const unsigned long long ob = (unsigned long long)__double_as_longlong(omega);
+    // omega * 2^-60 and -omega * 2^-8 by their exponents; an omega outside [2^-500, 2^500] goes the
+    // other way (tested on the exponent field: a comparison would be an FP64 instruction)
+    const bool plain_omega = (unsigned)(ob >> 52) - 523u <= 1000u;
+    const double om60 = __longlong_as_double((long long)(ob - (60ull << 52)));
+    const double omc = __longlong_as_double((long long)((ob - (8ull << 52)) ^ (1ull << 63)));
+    double g[9];
+    strict::Fixed m;
+    if (strict::fast_collide(f, g, om60, omc, m) && plain_omega) {
+#pragma unroll
+        for (int d = 0; d < 9; ++d) f[d] = g[d];
+        return { m.rho, m.jx, m.jy, m.usq122, true };
+    }
+    const Moments s = collide_f64_strict(f, omega);
+    return { __double_as_longlong(s.rho), __double_as_longlong(s.jx), __double_as_longlong(s.jy), s.usq, false };
+}
+
 template <int PREC>
-using MomentsOf = typename std::conditional<sizeof(typename Store<PREC>::C) == 4, MomentsF, Moments>::type;
+using MomentsOf = typename std::conditional<sizeof(typename Store<PREC>::C) == 4, MomentsF,
+                                            typename std::conditional<PREC == F64_STRICT, MomentsS, Moments>::type>::type;
 
 template <int PREC>
 __device__ __forceinline__ MomentsOf<PREC> collide(typename Store<PREC>::C f[9], const StepParams &p)
 {
-    if constexpr (PREC == F64_STRICT) return collide_f64_strict(f, p.omega);
+    if constexpr (PREC == F64_STRICT) return collide_strict(f, p.omega);
     else if constexpr (PREC == F64_FAST) return collide_f64_fast(f, p.omega);
     else if constexpr (PREC == F32_REF) return collide_f32_ref(f, p.omegaf);
     else if constexpr (PREC == F64_Q60) return collide_q60(f, p);
@@ -531,6 +559,11 @@ __device__ __forceinline__ void observables(const MomentsOf<PREC> &m, int xi, in
     if constexpr (PREC == F32_REF) {
         const Moments d = { (double)m.rho, (double)m.jx, (double)m.jy, (double)m.usq };
         write_observables_f32ref(d, xi, yi, p);
+    } else if constexpr (PREC == F64_STRICT) {
+        Moments d = { __longlong_as_double(m.rho), __longlong_as_double(m.jx), __longlong_as_double(m.jy), m.usq };
+        if (m.fixed)   // powers of two: exact
+            d = { (double)m.rho * 0x1p-61, (double)m.jx * 0x1p-61, (double)m.jy * 0x1p-61, m.usq * 0x1p-122 };
+        write_observables(d, xi, yi, p);
     } else if constexpr (PREC == F64_Q60) {
         const Moments d = { q_to_double(__double_as_longlong(m.rho)), q_to_double(__double_as_longlong(m.jx)),
                             q_to_double(__double_as_longlong(m.jy)), q_to_double(__double_as_longlong(m.usq)) };

@@ -3,8 +3,10 @@
 #include "plbm_kernels.cuh"
 
 #define PLBM_CASE(KER, PR, LA) case (PR) * 3 + (LA): KER<PR, LA><<<grid, block, 0, s>>>(p); break;
-#define PLBM_ALL_CASES(KER)                                                                   \
-    PLBM_CASE(KER, 0, 0) PLBM_CASE(KER, 0, 1) PLBM_CASE(KER, 0, 2)                             \
+#define PLBM_ALL_CASES(KER) PLBM_ALL_CASES_2(KER, KER)
+// STRICT: the kernel of the F64_STRICT form
+#define PLBM_ALL_CASES_2(STRICT, KER)                                                         \
+    PLBM_CASE(STRICT, 0, 0) PLBM_CASE(STRICT, 0, 1) PLBM_CASE(STRICT, 0, 2)                    \
     PLBM_CASE(KER, 1, 0) PLBM_CASE(KER, 1, 1) PLBM_CASE(KER, 1, 2)                             \
     PLBM_CASE(KER, 2, 0) PLBM_CASE(KER, 2, 1) PLBM_CASE(KER, 2, 2)                             \
     PLBM_CASE(KER, 3, 0) PLBM_CASE(KER, 3, 1) PLBM_CASE(KER, 3, 2)                             \

@@ -75,8 +75,11 @@ __device__ __forceinline__ void emit_observables(const MomentsOf<PREC> &m, int x
 // Launch bounds of the nptl, lptl and npol step kernels: the Q60 form runs 256-thread blocks and
 // is limited by memory latency, so it is held to 48 registers for a fifth resident block per SM
 // (measured faster despite a few spilled words; nsol measured equal and keeps its registers).
+// F64_STRICT takes 80 registers for three blocks: 4096 x 4096 16.2 k MLUPS against 14.7 k with two
+// (105 registers) and 15.8 k with four (64, spills).
 template <int PREC> struct NptlBounds { static constexpr int threads = 512, blocks = 1; };
 template <> struct NptlBounds<F64_Q60> { static constexpr int threads = 256, blocks = 5; };
+template <> struct NptlBounds<F64_STRICT> { static constexpr int threads = 256, blocks = 3; };
 
 // Collision (AoS) layout: the 32 nodes of a warp that lies in one row (or one run of the linear
 // index) own 32 consecutive records, 288 consecutive entries of the destination lattice.  Written
@@ -763,17 +766,17 @@ __device__ __forceinline__ void nsol_even_collision_staged(const StepParams &p)
 
 // The staged even step as its own kernel (launched by launch_nsol for 32 x NSOL_STAGE_ROWS blocks
 // in the collision layout): 256 threads, four resident blocks (the 64-register cap an unbounded
-// kernel gets), five for the Q60 form (48 registers, measured faster).  The other nsol kernels keep
-// no launch bounds: a bound above 256 threads let the compiler take 98 registers for the stream
+// kernel gets), five for the Q60 form (48 registers, measured faster), three for F64_STRICT.  The
+// other nsol kernels keep no launch bounds, except F64_STRICT's (three blocks of 256, 80 registers): a bound above 256 threads let the compiler take 98 registers for the stream
 // layout's even step and halved its resident blocks.
 template <int PREC>
-__global__ void __launch_bounds__(256, PREC == F64_Q60 ? 5 : 4) k_nsol_even_staged(StepParams p)
+__global__ void __launch_bounds__(256, PREC == F64_Q60 ? 5 : PREC == F64_STRICT ? 3 : 4) k_nsol_even_staged(StepParams p)
 {
     nsol_even_collision_staged<PREC>(p);
 }
 
 template <int PREC, int L>
-__global__ void k_nsol_even(StepParams p)
+__device__ __forceinline__ void nsol_even_step(const StepParams &p)
 {
     const int xi = blockIdx.x * blockDim.x + threadIdx.x;
     const int yi = blockIdx.y * blockDim.y + threadIdx.y;
@@ -828,8 +831,14 @@ __device__ __forceinline__ void nsol_odd_gather(CT<PREC> f[9], unsigned long lon
     }
 }
 
+template <int PREC, int L> __global__ void k_nsol_even(StepParams p) { nsol_even_step<PREC, L>(p); }
+template <int PREC, int L> __global__ void __launch_bounds__(256, 3) k_nsol_even_bound(StepParams p)
+{
+    nsol_even_step<PREC, L>(p);
+}
+
 template <int PREC, int L>
-__global__ void k_nsol_odd(StepParams p)
+__device__ __forceinline__ void nsol_odd_step(const StepParams &p)
 {
     const int xi = blockIdx.x * blockDim.x + threadIdx.x;
     const int yi = blockIdx.y * blockDim.y + threadIdx.y;
@@ -864,6 +873,12 @@ __global__ void k_nsol_odd(StepParams p)
 #pragma unroll
     for (int d = 0; d < 9; ++d) st<PREC>(p.lat0, lidx<L>(n, 8 - d, p.N), 8 - d, f[d], p);
     emit_observables<PREC>(m, xi, yi, p);
+}
+
+template <int PREC, int L> __global__ void k_nsol_odd(StepParams p) { nsol_odd_step<PREC, L>(p); }
+template <int PREC, int L> __global__ void __launch_bounds__(256, 3) k_nsol_odd_bound(StepParams p)
+{
+    nsol_odd_step<PREC, L>(p);
 }
 
 }  // namespace plbm

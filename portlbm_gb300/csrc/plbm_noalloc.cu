@@ -53,7 +53,7 @@ __global__ void k_nptl_noalloc(plbm::StepParams p, const int8_t *flags)
 #pragma unroll
     for (int d = 0; d < 9; ++d) f[d] = pull_one<F64_STRICT, STREAM>(p.lat0, n, xi, yi, d, lk, p);
     if (is_outlet_row(xi, yi, p)) outlet_fill<F64_STRICT>(f, jy_prev_at(p, yi), p);
-    const Moments m = collide<F64_STRICT>(f, p);
+    const MomentsS m = collide<F64_STRICT>(f, p);
 #pragma unroll
     for (int d = 0; d < 9; ++d) st<F64_STRICT>(p.lat1, lidx<STREAM>(n, d, p.N), d, f[d], p);
     observables<F64_STRICT>(m, xi, yi, p);
