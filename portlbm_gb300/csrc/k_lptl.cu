@@ -10,12 +10,10 @@ cudaError_t launch_lptl(int prec, int lay, const StepParams &p, dim3 grid, dim3 
             PLBM_POROUS_CASES(k_lptl)
         default: return cudaErrorInvalidValue;
         }
-        return cudaGetLastError();
     }
     switch (prec * 3 + lay) {
         PLBM_ALL_CASES(k_lptl)
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 }  // namespace plbm

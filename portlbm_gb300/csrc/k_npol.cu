@@ -9,6 +9,5 @@ cudaError_t launch_npol(int prec, int lay, const StepParams &p, dim3 grid, dim3 
         PLBM_ALL_CASES(k_npol)
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 }  // namespace plbm

@@ -10,29 +10,25 @@ cudaError_t launch_nptl(int prec, int lay, const StepParams &p, dim3 grid, dim3 
     // 2-byte storage in the stream layout on porous geometries: vectorised rows with the bounce-back
     // merged word-wise
     if (porous && two_byte && lay == STREAM) {
-        if (prec == F16S) k_nptl_vec_porous<F16S><<<vg, vb, 0, s>>>(p);
-        else if (prec == F16C) k_nptl_vec_porous<F16C><<<vg, vb, 0, s>>>(p);
-        else k_nptl_vec_porous<BF16S><<<vg, vb, 0, s>>>(p);
-        return cudaGetLastError();
+        if (prec == F16S) return launch_step_kernel(k_nptl_vec_porous<F16S>, vg, vb, s, p);
+        else if (prec == F16C) return launch_step_kernel(k_nptl_vec_porous<F16C>, vg, vb, s, p);
+        else return launch_step_kernel(k_nptl_vec_porous<BF16S>, vg, vb, s, p);
     }
     if (porous && ((prec >= F32 && prec <= BF16S) || prec == F16C)) {
         switch (prec * 3 + lay) {
             PLBM_POROUS_CASES(k_nptl)
         default: return cudaErrorInvalidValue;
         }
-        return cudaGetLastError();
     }
     // 2-byte storage in the stream layout: vectorised rows (launch shape of its own)
     if (two_byte && lay == STREAM) {
-        if (prec == F16S) k_nptl_vec<F16S><<<vg, vb, 0, s>>>(p);
-        else if (prec == F16C) k_nptl_vec<F16C><<<vg, vb, 0, s>>>(p);
-        else k_nptl_vec<BF16S><<<vg, vb, 0, s>>>(p);
-        return cudaGetLastError();
+        if (prec == F16S) return launch_step_kernel(k_nptl_vec<F16S>, vg, vb, s, p);
+        else if (prec == F16C) return launch_step_kernel(k_nptl_vec<F16C>, vg, vb, s, p);
+        else return launch_step_kernel(k_nptl_vec<BF16S>, vg, vb, s, p);
     }
     switch (prec * 3 + lay) {
         PLBM_ALL_CASES(k_nptl)
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 }  // namespace plbm

@@ -8,17 +8,16 @@ cudaError_t launch_nsol(int prec, int lay, const StepParams &p, unsigned t, dim3
     if ((t & 1u) == 0) {
         if (lay == COLLISION && block.x == 32 && block.y >= 1 && block.y <= (unsigned)NSOL_STAGE_ROWS) {
             switch (prec) {   // the record layout's even step with its stores staged per block
-            case 0: k_nsol_even_staged<0><<<grid, block, 0, s>>>(p); break;
-            case 1: k_nsol_even_staged<1><<<grid, block, 0, s>>>(p); break;
-            case 2: k_nsol_even_staged<2><<<grid, block, 0, s>>>(p); break;
-            case 3: k_nsol_even_staged<3><<<grid, block, 0, s>>>(p); break;
-            case 4: k_nsol_even_staged<4><<<grid, block, 0, s>>>(p); break;
-            case 5: k_nsol_even_staged<5><<<grid, block, 0, s>>>(p); break;
-            case 6: k_nsol_even_staged<6><<<grid, block, 0, s>>>(p); break;
-            case 7: k_nsol_even_staged<7><<<grid, block, 0, s>>>(p); break;
+            case 0: return launch_step_kernel(k_nsol_even_staged<0>, grid, block, s, p);
+            case 1: return launch_step_kernel(k_nsol_even_staged<1>, grid, block, s, p);
+            case 2: return launch_step_kernel(k_nsol_even_staged<2>, grid, block, s, p);
+            case 3: return launch_step_kernel(k_nsol_even_staged<3>, grid, block, s, p);
+            case 4: return launch_step_kernel(k_nsol_even_staged<4>, grid, block, s, p);
+            case 5: return launch_step_kernel(k_nsol_even_staged<5>, grid, block, s, p);
+            case 6: return launch_step_kernel(k_nsol_even_staged<6>, grid, block, s, p);
+            case 7: return launch_step_kernel(k_nsol_even_staged<7>, grid, block, s, p);
             default: return cudaErrorInvalidValue;
             }
-            return cudaGetLastError();
         }
         switch (prec * 3 + lay) {
             PLBM_ALL_CASES_2(k_nsol_even_bound, k_nsol_even)
@@ -30,6 +29,5 @@ cudaError_t launch_nsol(int prec, int lay, const StepParams &p, unsigned t, dim3
         default: return cudaErrorInvalidValue;
         }
     }
-    return cudaGetLastError();
 }
 }  // namespace plbm

@@ -2,11 +2,28 @@
 #pragma once
 #include "plbm_kernels.cuh"
 
-#define PLBM_CASE(KER, PR, LA) case (PR) * 3 + (LA): KER<PR, LA><<<grid, block, 0, s>>>(p); break;
+namespace plbm {
+// Launches a step kernel (one that calls step_begin) with programmatic stream serialization.
+inline cudaError_t launch_step_kernel(void (*kernel)(StepParams), dim3 grid, dim3 block, cudaStream_t s, const StepParams &p)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+}  // namespace plbm
+
+#define PLBM_CASE(KER, PR, LA) case (PR) * 3 + (LA): return launch_step_kernel(KER<PR, LA>, grid, block, s, p);
 #define PLBM_ALL_CASES(KER) PLBM_ALL_CASES_2(KER, KER)
-// STRICT: the kernel of the F64_STRICT form
-#define PLBM_ALL_CASES_2(STRICT, KER)                                                         \
-    PLBM_CASE(STRICT, 0, 0) PLBM_CASE(STRICT, 0, 1) PLBM_CASE(STRICT, 0, 2)                    \
+// BOUND: the kernel of the F64_STRICT form
+#define PLBM_ALL_CASES_2(BOUND, KER)                                                          \
+    PLBM_CASE(BOUND, 0, 0) PLBM_CASE(BOUND, 0, 1) PLBM_CASE(BOUND, 0, 2)                       \
     PLBM_CASE(KER, 1, 0) PLBM_CASE(KER, 1, 1) PLBM_CASE(KER, 1, 2)                             \
     PLBM_CASE(KER, 2, 0) PLBM_CASE(KER, 2, 1) PLBM_CASE(KER, 2, 2)                             \
     PLBM_CASE(KER, 3, 0) PLBM_CASE(KER, 3, 1) PLBM_CASE(KER, 3, 2)                             \
@@ -16,7 +33,7 @@
     PLBM_CASE(KER, 7, 0) PLBM_CASE(KER, 7, 1) PLBM_CASE(KER, 7, 2)
 
 // The porous gather of the shifted forms (f32, f16s, bf16s, f16c; the unshifted forms have one gather).
-#define PLBM_POROUS_CASE(KER, PR, LA) case (PR) * 3 + (LA): KER<PR, LA, true><<<grid, block, 0, s>>>(p); break;
+#define PLBM_POROUS_CASE(KER, PR, LA) case (PR) * 3 + (LA): return launch_step_kernel(KER<PR, LA, true>, grid, block, s, p);
 #define PLBM_POROUS_CASES(KER)                                                                \
     PLBM_POROUS_CASE(KER, 3, 0) PLBM_POROUS_CASE(KER, 3, 1) PLBM_POROUS_CASE(KER, 3, 2)        \
     PLBM_POROUS_CASE(KER, 4, 0) PLBM_POROUS_CASE(KER, 4, 1) PLBM_POROUS_CASE(KER, 4, 2)        \

@@ -151,7 +151,8 @@ template <int PREC> struct RowsPerThread { static constexpr int value = rows_per
 //    neighbours, pull_one for the rest (open channels).
 // STAGED (collision layout, NY == 1, called by whole warps whose 32 nodes are consecutive):
 // the destination records are written through store_records_staged.
-template <int PREC, int L, int NY, bool POROUS = false, bool STAGED = false>
+// STEP: called by a step kernel, once (step_begin after the link words are loaded).
+template <int PREC, int L, int NY, bool POROUS = false, bool STAGED = false, bool STEP = false>
 __device__ __forceinline__ void update_two_lattice_rows(const int xi[NY], const int yi[NY], const StepParams &p)
 {
     static_assert(!STAGED || (L == COLLISION && NY == 1), "staged stores: collision layout, one node per thread");
@@ -165,6 +166,7 @@ __device__ __forceinline__ void update_two_lattice_rows(const int xi[NY], const 
         n[j] = in ? (unsigned long long)xi[j] + (unsigned long long)yi[j] * p.P : 0;
         lk[j] = in ? link_at(p, n[j]) : 0;
     }
+    if constexpr (STEP) step_begin();
 #pragma unroll
     for (int j = 0; j < NY; ++j) {
         const bool interior = (lk[j] & (LINK_FLUID | LINK_EDGE)) == LINK_FLUID;
@@ -201,6 +203,7 @@ __device__ __forceinline__ void update_two_lattice_rows(const int xi[NY], const 
             if (is_outlet_row(xi[0], yi[0], p)) outlet_fill<PREC>(f[0], jy_prev_at(p, yi[0]), p);
             m = collide<PREC>(f[0], p);
         }
+        if constexpr (STEP) step_collided();
         store_records_staged<PREC>(p, p.lat1, n[0], f[0], fluid);
         if (fluid) emit_observables<PREC>(m, xi[0], yi[0], p);
     } else {
@@ -217,6 +220,7 @@ __device__ __forceinline__ void update_two_lattice_rows(const int xi[NY], const 
             }
             if (is_outlet_row(xi[j], yi[j], p)) outlet_fill<PREC>(f[j], jy_prev_at(p, yi[j]), p);
             const auto m = collide<PREC>(f[j], p);
+            if constexpr (STEP) step_collided();
 #pragma unroll
             for (int d = 0; d < 9; ++d) st<PREC>(p.lat1, lidx<L>(n[j], d, p.N), d, f[j][d], p);
             emit_observables<PREC>(m, xi[j], yi[j], p);
@@ -239,7 +243,7 @@ __global__ void __launch_bounds__(NptlBounds<PREC>::threads, NptlBounds<PREC>::b
             // padded row; lanes past W take part in the staged store as non-fluid nodes
             if (y0 >= p.H || x - (int)(threadIdx.x & 31u) >= p.P) return;
             const int xs[1] = { x }, ys[1] = { y0 };
-            update_two_lattice_rows<PREC, L, 1, POROUS, true>(xs, ys, p);
+            update_two_lattice_rows<PREC, L, 1, POROUS, true, true>(xs, ys, p);
             return;
         }
     }
@@ -247,7 +251,7 @@ __global__ void __launch_bounds__(NptlBounds<PREC>::threads, NptlBounds<PREC>::b
     int xi[NY], yi[NY];
 #pragma unroll
     for (int j = 0; j < NY; ++j) { xi[j] = x; yi[j] = y0 + j; }
-    update_two_lattice_rows<PREC, L, NY, POROUS>(xi, yi, p);
+    update_two_lattice_rows<PREC, L, NY, POROUS, false, true>(xi, yi, p);
 }
 
 // nptl, stream layout, 2-byte storage (F16S / BF16S): each thread updates VEC consecutive nodes
@@ -336,6 +340,7 @@ __device__ __forceinline__ void vec_row_segment(const StepParams &p, int y, int 
     unsigned r[9][4];
     const uint4 l4 = in_range(row0 + x0 + VEC - 1, p.N, p) ? *reinterpret_cast<const uint4 *>(p.links + row0 + x0)
                                                          : make_uint4(0, 0, 0, 0);
+    step_begin();
     if (inner_row) {
 #pragma unroll
         for (int d = 0; d < 9; ++d) {   // all nine loads are issued before any is used
@@ -427,6 +432,7 @@ __device__ __forceinline__ void vec_row_segment_porous(const StepParams &p, int 
     // bits 0-3 and 5-8 of both halves: a solid source (bit 4 marks fluid)
     const bool bounce_here = ((lw[0] | lw[1] | lw[2] | lw[3]) & 0x01EF01EFu) != 0;
     const bool bounce_warp = __any_sync(0xffffffffu, inner_row && bounce_here);
+    step_begin();
     if (inner_row) {
         unsigned o[6][4];   // own row of planes 0, 1, 2, 6, 7, 8
 #pragma unroll
@@ -572,10 +578,10 @@ __global__ void __launch_bounds__(NptlBounds<PREC>::threads, NptlBounds<PREC>::b
     }
     if constexpr (L == COLLISION && NY == 1) {
         // blockDim.x is a multiple of 32: every warp covers 32 consecutive linear indices
-        update_two_lattice_rows<PREC, L, 1, POROUS, true>(xi, yi, p);
+        update_two_lattice_rows<PREC, L, 1, POROUS, true, true>(xi, yi, p);
         return;
     }
-    update_two_lattice_rows<PREC, L, NY, POROUS>(xi, yi, p);
+    update_two_lattice_rows<PREC, L, NY, POROUS, false, true>(xi, yi, p);
 }
 
 // ---- npol: in place, one tile per thread block --------------------------------------------
@@ -607,6 +613,7 @@ __global__ void __launch_bounds__(NptlBounds<PREC>::threads, NptlBounds<PREC>::b
     const uint16_t lk = inside ? link_at(p, n) : 0;
     const bool fluid = (lk & LINK_FLUID) != 0;
     const int lx = threadIdx.x, ly = threadIdx.y;
+    step_begin();
     CT<PREC> f[9];
     if (fluid) {
         if (lk == LINK_FLUID) {
@@ -737,6 +744,7 @@ __device__ __forceinline__ void nsol_even_collision_staged(const StepParams &p)
     const bool inside = xi < p.W && yi < p.H;
     const unsigned long long n = inside ? (unsigned long long)xi + (unsigned long long)yi * p.P : 0;
     const uint16_t lk = inside ? link_at(p, n) : 0;
+    step_begin();
     if (lk & LINK_FLUID) {
         CT<PREC> f[9];
         nsol_even_gather<PREC, COLLISION>(f, n, xi, yi, lk, p);
@@ -783,6 +791,7 @@ __device__ __forceinline__ void nsol_even_step(const StepParams &p)
     if (xi >= p.W || yi >= p.H) return;
     const unsigned long long n = (unsigned long long)xi + (unsigned long long)yi * p.P;
     const uint16_t lk = link_at(p, n);
+    step_begin();
     if (!(lk & LINK_FLUID)) return;
     CT<PREC> f[9];
     nsol_even_gather<PREC, L>(f, n, xi, yi, lk, p);
@@ -849,6 +858,7 @@ __device__ __forceinline__ void nsol_odd_step(const StepParams &p)
             const bool in = xi < p.W;
             const unsigned long long n = in ? (unsigned long long)xi + (unsigned long long)yi * p.P : 0;
             const uint16_t lk = in ? link_at(p, n) : 0;
+            step_begin();
             const bool fluid = (lk & LINK_FLUID) != 0;
             CT<PREC> f[9];
             MomentsOf<PREC> m{};
@@ -865,6 +875,7 @@ __device__ __forceinline__ void nsol_odd_step(const StepParams &p)
     if (xi >= p.W || yi >= p.H) return;
     const unsigned long long n = (unsigned long long)xi + (unsigned long long)yi * p.P;
     const uint16_t lk = link_at(p, n);
+    step_begin();
     if (!(lk & LINK_FLUID)) return;
     CT<PREC> f[9];
     nsol_odd_gather<PREC, L>(f, n, xi, yi, lk, p);
