@@ -189,7 +189,8 @@ int plbm_write_npy(const char *path, const double *data, unsigned rows, unsigned
 int plbm_benchmark_run(const char *settings_path, const char *benchmark_path, const char *output_root,
                        const plbm_options *opts, unsigned phases, double hbm_gbs);
 int plbm_benchmark_work_group_sizes(unsigned max_work_group_size, unsigned *out, unsigned capacity, unsigned *count);
-/* Kernel launches issued per step (for launch accounting). */
+/* Kernel launches issued per step (for launch accounting); plain steps of the shifted forms on large
+ * nptl / lptl domains run two a launch. */
 int plbm_launches_per_step(plbm_handler *h, unsigned *n);
 /* Algorithmic HBM bytes per node update of the hot kernel (9 loads + 9 stores). */
 int plbm_bytes_per_node(plbm_handler *h, double *bytes);

@@ -1,0 +1,38 @@
+// k_pair.cu — instantiations of the two-step kernel of nptl and lptl.
+#include "plbm_dispatch.cuh"
+#include "plbm_launch.h"
+#include "plbm_pair.cuh"
+
+namespace plbm {
+
+template <int PREC, int L>
+static cudaError_t launch(const StepParams &p, int rows, cudaStream_t s)
+{
+    const int strips = (p.W + PAIR_COLUMNS - 1) / PAIR_COLUMNS;
+    const dim3 grid((unsigned)((strips + PAIR_WARPS - 1) / PAIR_WARPS), (unsigned)((p.H + rows - 1) / rows));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(32, PAIR_WARPS);
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_two_steps<PREC, L>, p, rows);
+}
+
+#define PLBM_PAIR_CASE(PR, LA) case (PR) * 3 + (LA): return launch<PR, LA>(p, rows, s);
+cudaError_t launch_two_steps(int prec, int lay, const StepParams &p, int rows, cudaStream_t s)
+{
+    switch (prec * 3 + lay) {
+        PLBM_PAIR_CASE(F32, 0) PLBM_PAIR_CASE(F32, 1) PLBM_PAIR_CASE(F32, 2)
+        PLBM_PAIR_CASE(F16S, 0) PLBM_PAIR_CASE(F16S, 1) PLBM_PAIR_CASE(F16S, 2)
+        PLBM_PAIR_CASE(BF16S, 0) PLBM_PAIR_CASE(BF16S, 1) PLBM_PAIR_CASE(BF16S, 2)
+        PLBM_PAIR_CASE(F16C, 0) PLBM_PAIR_CASE(F16C, 1) PLBM_PAIR_CASE(F16C, 2)
+        PLBM_PAIR_CASE(F64_Q60, 0) PLBM_PAIR_CASE(F64_Q60, 1) PLBM_PAIR_CASE(F64_Q60, 2)
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace plbm

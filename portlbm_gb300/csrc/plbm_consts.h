@@ -80,6 +80,16 @@ inline void fill_float_constants(StepParams &b, bool shifted, bool profile, doub
         b.shift_cx[d] = (float)(w * g * cx * scale);
     }
     b.omegaf = (float)b.omega;
+    const float qs = 1.0f / (float)scale;
+    b.c_om1 = 1.0f - b.omegaf;
+    b.c_ow9 = b.omegaf * (1.0f / 9);
+    b.c_ow36 = b.omegaf * (1.0f / 36);
+    b.c_ow49 = b.omegaf * (4.0f / 9);
+    b.c_k9 = 4.5f * b.c_ow9 * qs;
+    b.c_k36 = 4.5f * b.c_ow36 * qs;
+    b.c_o9 = 3.0f * b.c_ow9;
+    b.c_o36 = 3.0f * b.c_ow36;
+    b.c_r = -1.5f * qs;
     // outlet: f1+f4+f7+2(f8+f5+f2) carries exactly 1 in rest weights, so xv = (rho0 - rho_out) + sum(df)
     b.rho_outf = shifted ? (float)((b.rho_out - r_out) * scale) : (float)b.rho_out;
 }

@@ -456,6 +456,8 @@ struct plbm_handler {
     int outlet_mode = 0;
     // debugMode on nptl / lptl: the reference's unfused stream / observables / collide kernels
     bool debug = false;
+    int pair_rows = 0;     // rows a warp of the two-step kernel marches over; 0: one step a launch
+    bool vec_rows = false; // nptl, 2-byte storage, stream layout: vectorised rows
     bool porous = false;   // nptl/lptl shifted forms: the obstacle-select gather (PLBM_GATHER_POROUS)
 
     cudaStream_t stream = nullptr;
@@ -843,6 +845,7 @@ struct plbm_handler {
             cuda_check(cudaMemcpy(&bad, status_d, sizeof(int), cudaMemcpyDeviceToHost), "mask check");
             if (bad) fail(PLBM_ERR_ARGUMENT, "mask entries must be 0 (fluid) or 1 (solid)");
         }
+        choose_kernels();
         trace("ready");
     }
 
@@ -861,11 +864,63 @@ struct plbm_handler {
         if (alg == 2) { p.halo_in = (double *)halo[par]; p.halo_out = (double *)halo[par ^ 1u]; }
         if (debug) return plbm::launch_debug_step(prec, lay, alg == 1, p, block, stream);
         switch (alg) {
-        case 0: return plbm::launch_nptl(prec, lay, p, grid, block, stream, porous);
+        case 0: return plbm::launch_nptl(prec, lay, p, grid, block, stream, porous, vec_rows);
         case 1: return plbm::launch_lptl(prec, lay, p, grid, block, stream, porous);
         case 2: return plbm::launch_npol(prec, lay, p, grid, block, stream);
         default: return plbm::launch_nsol(prec, lay, p, t, grid, block, stream);
         }
+    }
+
+    // The kernels of nptl and lptl that pay on domains whose two lattices outgrow L2:
+    //  * plain steps two a launch.  Shifted forms from half of L2 on: f32 72 MB of lattices 10.7 us a step
+    //    singly against 10.5, 111 MB 19.4 / 14.6, 216 MB 38.1 / 27.0; f16s 72 MB 20.6 / 19.5, 108 MB
+    //    36.3 / 27.3; below (1000 x 300) 4.6 / 5.4.  F64_Q60, bound by instructions as much as by HBM,
+    //    from eight times L2 on: 1.2 GB 180 / 173, 2.4 GB 433 / 373, but 144 MB 26.2 / 30.5.  The rows of
+    //    a strip trade rows done twice against blocks enough for every SM: shifted 4 up to 4 M nodes
+    //    (3 M: 27.0, with 8 rows 28.0), 8 up to 32 M (8 M: 59.9, with 4 rows 61.6), 16 above (67 M: 429,
+    //    with 8 rows 445); Q60 16 up to 16 M, 32 above (67 M: 1222, with 16 rows 1254).
+    //  * nptl's 2-byte forms step vectorised rows in the stream layout from four fifths of L2 on; on
+    //    smaller domains, where the few warps of 256 nodes wait, the scalar kernel (1000 x 300 f16s 9.3
+    //    against 6.0 us, 2000 x 500 14.3 / 11.3, 3000 x 1000 32.8 / 34.1).
+    void choose_kernels()
+    {
+        int l2 = 0;
+        cuda_check(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, opt.device), "device attribute");
+        const unsigned long long lattices = 2 * 9ull * N * storage_bytes(prec), cache = (unsigned long long)l2;
+        const bool shifted = prec == PLBM_F32 || prec == PLBM_F16S || prec == PLBM_BF16S || prec == PLBM_F16C;
+        vec_rows = lattices > cache / 5 * 4;
+        pair_rows = 0;
+        if (!two_lattice() || debug) return;
+        if (shifted && lattices > cache / 2) pair_rows = N < (1ull << 22) ? 4 : N < (1ull << 25) ? 8 : 16;
+        if (prec == PLBM_F64_Q60 && lattices > 8 * cache) pair_rows = N < (1ull << 24) ? 16 : 32;
+        // the kernel's offsets (bytes, values of 8-byte storage) and its grid height are 32 and 16 bits
+        const unsigned long long offsets = 9ull * N * (prec == PLBM_F64_Q60 ? 1 : storage_bytes(prec));
+        if (pair_rows && (offsets >= (1ull << 32) || (H + pair_rows - 1) / pair_rows > 65535)) pair_rows = 0;
+    }
+
+    // Two steps in one launch, without results: the state of lat[par] goes to lat[par ^ 1].
+    cudaError_t launch_two_steps(unsigned par)
+    {
+        plbm::StepParams p = base;
+        p.write_results = 0;
+        p.lat0 = lat[par];
+        p.lat1 = lat[par ^ 1u];
+        p.jy_prev = jy_d + (size_t)par * H;
+        p.jy_next = jy_d + (size_t)(par ^ 1u) * H;
+        return plbm::launch_two_steps(prec, lay, p, pair_rows, stream);
+    }
+
+    // Enqueues n steps from step t without results: four at a time in two two-step launches, so that
+    // step t's state stays in lat[t & 1], the rest one by one.
+    cudaError_t enqueue_plain(unsigned t, unsigned n)
+    {
+        cudaError_t e = cudaSuccess;
+        for (; pair_rows && n >= 4 && e == cudaSuccess; t += 4, n -= 4) {
+            e = launch_two_steps(t & 1u);
+            if (e == cudaSuccess) e = launch_two_steps((t & 1u) ^ 1u);
+        }
+        for (; n > 0 && e == cudaSuccess; ++t, --n) e = launch_step(t, false);
+        return e;
     }
 
     // Captures `pairs` (even, odd) step pairs without result writes into one executable graph.
@@ -875,8 +930,7 @@ struct plbm_handler {
         const unsigned pairs = N >= (1ull << 22) ? 4 : 32;
         cudaGraph_t g = nullptr;
         cuda_check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-        cudaError_t e = cudaSuccess;
-        for (unsigned k = 0; k < 2 * pairs && e == cudaSuccess; ++k) e = launch_step(k, false);
+        const cudaError_t e = enqueue_plain(0, 2 * pairs);
         cudaError_t e2 = cudaStreamEndCapture(stream, &g);
         cuda_check(e, "capture launch");
         cuda_check(e2, "end capture");
@@ -899,8 +953,8 @@ struct plbm_handler {
         wait_host();   // the copies target the pinned host arrays
         cudaGraph_t g = nullptr;
         cuda_check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-        cudaError_t e = cudaSuccess;
-        for (unsigned k = 0; k < F && e == cudaSuccess; ++k) e = launch_step(t0 + k, k + 1 == F, k + 1 == F);
+        cudaError_t e = enqueue_plain(t0, F - 1);
+        if (e == cudaSuccess) e = launch_step(t0 + F - 1, true, true);
         cudaError_t e2 = cudaStreamEndCapture(stream, &g);
         cuda_check(e, "frame capture");
         cuda_check(e2, "end capture");
@@ -921,7 +975,7 @@ struct plbm_handler {
                 t += graph_steps;
             }
         }
-        for (; t < t1; ++t) cuda_check(launch_step(t, false), "step");
+        cuda_check(enqueue_plain(t, t1 - t), "step");
     }
 
     // The Q60 form records a population that left its fixed-point range in a device word.
@@ -1362,6 +1416,7 @@ int plbm_set_precision(plbm_handler *h, int precision)
         for (int i = 0; i < 2 && hn; ++i) { cudaFree(h->halo[i]); h->halo[i] = nhalo[i]; nhalo[i] = nullptr; }
         h->base = b;
         h->prec = precision;
+        h->choose_kernels();
         if (h->gexec) cudaGraphExecDestroy(h->gexec);
         h->gexec = nullptr;
         h->graph_steps = 0;

@@ -9,8 +9,13 @@ namespace plbm {
 // One timestep of algorithm `alg` (0 nptl, 1 lptl, 2 npol, 3 nsol) for precision `prec` and
 // layout `lay`; `t` is the absolute step index (selects the nsol parity kernel).
 // porous: the obstacle-select gather of the shifted forms (f32, f16s, bf16s)
-cudaError_t launch_nptl(int prec, int lay, const StepParams &p, dim3 grid, dim3 block, cudaStream_t s, bool porous);
+// vec_rows: the vectorised rows of the 2-byte forms (stream layout)
+cudaError_t launch_nptl(int prec, int lay, const StepParams &p, dim3 grid, dim3 block, cudaStream_t s, bool porous,
+                        bool vec_rows);
 cudaError_t launch_lptl(int prec, int lay, const StepParams &p, dim3 grid, dim3 block, cudaStream_t s, bool porous);
+// Two timesteps of nptl / lptl in one launch: reads p.lat0, writes the state after both to p.lat1 (no
+// results).  rows: rows of the domain a warp marches over.
+cudaError_t launch_two_steps(int prec, int lay, const StepParams &p, int rows, cudaStream_t s);
 // counts[0] = 32-node row segments holding fluid, counts[1] = those mixing interior nodes with and
 // without a solid neighbour
 cudaError_t launch_count_obstacle_nodes(const uint16_t *links, int W, int H, int P, unsigned long long *counts,

@@ -64,6 +64,9 @@ struct StepParams {
     // would run on the FP64 pipe)
     float feq_inf[9], feq_outf[9], weightf[9];
     float omegaf, rho_outf;
+    // coefficients of the FP32 collision, rounded as the products it would form: 1 - omega, omega w_d,
+    // 4.5 omega w_d / scale, 3 omega w_d, and 1.5 / scale (scale: F16_SCALE for the FP16 form, else 1)
+    float c_om1, c_ow49, c_ow9, c_ow36, c_k9, c_k36, c_o9, c_o36, c_r;
     // Shifted forms (F32, F16S, BF16S) hold f_d - w_d * rho0(x') with rho0(x') = shift_a - shift_g * x'.
     // Two-lattice pull schemes use the straight profile between the inlet ghost column (x' = -1,
     // rho_in) and the outlet ghost column (x' = W, rho_out); the others use rho0 = 1.  Every
