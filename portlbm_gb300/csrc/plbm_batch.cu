@@ -95,7 +95,7 @@ __device__ __forceinline__ void vec_edge_column(float *f, int x, int y, const St
     if (x == p.W - 1) {
         f[0] = g_out<PREC>(p, 0); f[3] = g_out<PREC>(p, 3); f[6] = g_out<PREC>(p, 6);
     }
-    if (is_outlet_row(x, y, p)) outlet_fill<PREC>(f, jy_prev_at(p, y), p);
+    if (is_outlet_row(x, y, p)) outlet_fill<PREC, true>(f, jy_prev_at(p, y), p);
 }
 
 // The porous row update of vec_row_segment_porous with the domain walked in row-major order
@@ -191,21 +191,21 @@ __device__ __forceinline__ void vec_linear_segment_porous(const StepParams &p, l
         const bool live_a = vec_ok && xa < p.W && (la & LINK_FLUID), live_b = vec_ok && xb < p.W && (lb & LINK_FLUID);
         if (live_a && (la & LINK_EDGE)) {
             if (inner_row) vec_edge_column<PREC>(fa, xa, y, p);
-            else vec_edge_gather<PREC>(fa, xa, y, la, p);
+            else vec_edge_gather<PREC, true>(fa, xa, y, la, p);
         }
         if (live_b && (lb & LINK_EDGE)) {
             if (inner_row) vec_edge_column<PREC>(fb, xb, y, p);
-            else vec_edge_gather<PREC>(fb, xb, y, lb, p);
+            else vec_edge_gather<PREC, true>(fb, xb, y, lb, p);
         }
         if (live_a) {
-            const MomentsF m = collide<PREC>(fa, p);
+            const MomentsF m = collide<PREC, true>(fa, p);
             emit_observables<PREC>(m, xa, y, p);
         } else {
 #pragma unroll
             for (int d = 0; d < 9; ++d) fa[d] = 0.0f;
         }
         if (live_b) {
-            const MomentsF m = collide<PREC>(fb, p);
+            const MomentsF m = collide<PREC, true>(fb, p);
             emit_observables<PREC>(m, xb, y, p);
         } else {
 #pragma unroll

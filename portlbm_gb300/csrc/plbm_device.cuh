@@ -297,27 +297,39 @@ __device__ __forceinline__ MomentsF collide_f32_ref(float f[9], float omega)
     return { rho, jx, jy, usq };
 }
 
-// FP32 arithmetic for the F32 / F16S / BF16S storage forms (same regrouping as F64_FAST), the
-// coefficients from the step parameters.  The FP16 form collides df * F16_SCALE: the update is linear
-// in f except for the two quadratic terms, whose coefficients take 1 / F16_SCALE.
-__device__ __forceinline__ MomentsF collide_f32(float f[9], const StepParams &p)
+// The coefficients of collide_f32: from the step parameters, operands in constant memory; or formed for
+// the node from omega (the same products), for the batch kernels, whose parameters lie in shared memory
+// (k_batch_vec<F16S> on 20 domains 87.8 us a step, 93.4 with the coefficients read).
+struct CoefficientsF { float om1, ow49, ow9, ow36, k9, k36, o9, o36, r; };
+template <bool FORMED> __device__ __forceinline__ CoefficientsF coefficients(const StepParams &p, float qs)
+{
+    if (!FORMED) return { p.c_om1, p.c_ow49, p.c_ow9, p.c_ow36, p.c_k9, p.c_k36, p.c_o9, p.c_o36, p.c_r };
+    const float ow9 = p.omegaf * (1.0f / 9), ow36 = p.omegaf * (1.0f / 36);
+    return { 1.0f - p.omegaf, p.omegaf * (4.0f / 9), ow9, ow36, 4.5f * ow9 * qs, 4.5f * ow36 * qs, 3.0f * ow9, 3.0f * ow36,
+             -1.5f * qs };
+}
+
+// FP32 arithmetic for the F32 / F16S / BF16S storage forms (same regrouping as F64_FAST).  The FP16
+// form collides df * F16_SCALE: the update is linear in f except for the two quadratic terms, whose
+// coefficients take 1 / F16_SCALE.
+__device__ __forceinline__ MomentsF collide_f32(float f[9], const CoefficientsF &c)
 {
     const float A = f[2] + f[5] + f[8], B = f[0] + f[3] + f[6];
     const float C = f[6] + f[7] + f[8], E = f[0] + f[1] + f[2];
     const float rho = (B + (f[1] + f[4] + f[7])) + A;
     const float jx = A - B, jy = C - E;
     const float usq = fmaf(jx, jx, jy * jy);
-    const float R = fmaf(p.c_r, usq, rho);
-    const float b9 = p.c_ow9 * R, b36 = p.c_ow36 * R;
-    f[4] = fmaf(p.c_om1, f[4], p.c_ow49 * R);
-    { const float u = jx, sym = fmaf(p.c_k9 * u, u, b9);
-      f[5] = fmaf(p.c_o9, u, fmaf(p.c_om1, f[5], sym)); f[3] = fmaf(-p.c_o9, u, fmaf(p.c_om1, f[3], sym)); }
-    { const float u = jy, sym = fmaf(p.c_k9 * u, u, b9);
-      f[7] = fmaf(p.c_o9, u, fmaf(p.c_om1, f[7], sym)); f[1] = fmaf(-p.c_o9, u, fmaf(p.c_om1, f[1], sym)); }
-    { const float u = jx + jy, sym = fmaf(p.c_k36 * u, u, b36);
-      f[8] = fmaf(p.c_o36, u, fmaf(p.c_om1, f[8], sym)); f[0] = fmaf(-p.c_o36, u, fmaf(p.c_om1, f[0], sym)); }
-    { const float u = jx - jy, sym = fmaf(p.c_k36 * u, u, b36);
-      f[2] = fmaf(p.c_o36, u, fmaf(p.c_om1, f[2], sym)); f[6] = fmaf(-p.c_o36, u, fmaf(p.c_om1, f[6], sym)); }
+    const float R = fmaf(c.r, usq, rho);
+    const float b9 = c.ow9 * R, b36 = c.ow36 * R;
+    f[4] = fmaf(c.om1, f[4], c.ow49 * R);
+    { const float u = jx, sym = fmaf(c.k9 * u, u, b9);
+      f[5] = fmaf(c.o9, u, fmaf(c.om1, f[5], sym)); f[3] = fmaf(-c.o9, u, fmaf(c.om1, f[3], sym)); }
+    { const float u = jy, sym = fmaf(c.k9 * u, u, b9);
+      f[7] = fmaf(c.o9, u, fmaf(c.om1, f[7], sym)); f[1] = fmaf(-c.o9, u, fmaf(c.om1, f[1], sym)); }
+    { const float u = jx + jy, sym = fmaf(c.k36 * u, u, b36);
+      f[8] = fmaf(c.o36, u, fmaf(c.om1, f[8], sym)); f[0] = fmaf(-c.o36, u, fmaf(c.om1, f[0], sym)); }
+    { const float u = jx - jy, sym = fmaf(c.k36 * u, u, b36);
+      f[2] = fmaf(c.o36, u, fmaf(c.om1, f[2], sym)); f[6] = fmaf(-c.o36, u, fmaf(c.om1, f[6], sym)); }
     return { rho, jx, jy, usq };
 }
 
@@ -486,14 +498,15 @@ template <int PREC>
 using MomentsOf = typename std::conditional<sizeof(typename Store<PREC>::C) == 4, MomentsF,
                                             typename std::conditional<PREC == F64_STRICT, MomentsS, Moments>::type>::type;
 
-template <int PREC>
+// FORMED: see CoefficientsF.
+template <int PREC, bool FORMED = false>
 __device__ __forceinline__ MomentsOf<PREC> collide(typename Store<PREC>::C f[9], const StepParams &p)
 {
     if constexpr (PREC == F64_STRICT) return collide_strict(f, p.omega);
     else if constexpr (PREC == F64_FAST) return collide_f64_fast(f, p.omega);
     else if constexpr (PREC == F32_REF) return collide_f32_ref(f, p.omegaf);
     else if constexpr (PREC == F64_Q60) return collide_q60(f, p);
-    else return collide_f32(f, p);
+    else return collide_f32(f, coefficients<FORMED>(p, PREC == F16S ? 1.0f / F16_SCALE : 1.0f));
 }
 
 // (float)(jyo * k), k a power of two.  A function of its own: inline, the compiler predicates these two
@@ -515,7 +528,9 @@ __device__ __forceinline__ void outlet_fill_float(float f[9], float hy, const St
 // Outlet populations 0, 3, 6 of a border node (X-2, y), y in [2, V-3], from its other pulled
 // values: OutletUpdateKernel non_buffered.hpp:95-129 with f_1 = f[1], f_4 = f[4], f_7 = f[7]
 // and f_inverse = {f[8], f[5], f[2]} (the same lattice entries).
-template <int PREC>
+// BATCH: in a batch kernel, where half_jy's call costs more than it saves (k_batch_vec<F16S> 90.3 us a
+// step on 20 domains against 87.6).
+template <int PREC, bool BATCH = false>
 __device__ __forceinline__ void outlet_fill(typename Store<PREC>::C f[9], double jyo, const StepParams &p)
 {
     if constexpr (PREC == F64_STRICT) {
@@ -546,7 +561,8 @@ __device__ __forceinline__ void outlet_fill(typename Store<PREC>::C f[9], double
         f[3] = (float)__dsub_rn((double)g1, __dmul_rn(2.0 / 3, (double)xv));
         f[6] = (float)__dadd_rn(__dsub_rn(__dadd_rn((double)g2, hd), x6), hy);
     } else if constexpr (sizeof(typename Store<PREC>::C) == 4) {
-        outlet_fill_float(f, half_jy(jyo, PREC == F16S ? 0.5 * F16_SCALE : 0.5), p);
+        constexpr double half = PREC == F16S ? 0.5 * F16_SCALE : 0.5;
+        outlet_fill_float(f, BATCH ? (float)(jyo * half) : half_jy(jyo, half), p);
     } else {
         using C = typename Store<PREC>::C;
         const C xv = -p.rho_outf + ((f[1] + f[4] + f[7]) + (C)2 * (f[8] + f[5] + f[2]));

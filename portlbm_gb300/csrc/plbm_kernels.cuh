@@ -151,7 +151,8 @@ template <int PREC> struct RowsPerThread { static constexpr int value = rows_per
 //    neighbours, pull_one for the rest (open channels).
 // STAGED (collision layout, NY == 1, called by whole warps whose 32 nodes are consecutive):
 // the destination records are written through store_records_staged.
-// STEP: called by a step kernel, once (step_begin after the link words are loaded).
+// STEP: called by a step kernel, once (step_begin after the link words are loaded); otherwise by a batch
+// kernel.
 template <int PREC, int L, int NY, bool POROUS = false, bool STAGED = false, bool STEP = false>
 __device__ __forceinline__ void update_two_lattice_rows(const int xi[NY], const int yi[NY], const StepParams &p)
 {
@@ -200,8 +201,8 @@ __device__ __forceinline__ void update_two_lattice_rows(const int xi[NY], const 
                         if (cxd(d) != 0 && !((lk[0] >> d) & 1u)) f[0][d] += p.shift_cx[d];
                 }
             }
-            if (is_outlet_row(xi[0], yi[0], p)) outlet_fill<PREC>(f[0], jy_prev_at(p, yi[0]), p);
-            m = collide<PREC>(f[0], p);
+            if (is_outlet_row(xi[0], yi[0], p)) outlet_fill<PREC, !STEP>(f[0], jy_prev_at(p, yi[0]), p);
+            m = collide<PREC, !STEP>(f[0], p);
         }
         if constexpr (STEP) step_collided();
         store_records_staged<PREC>(p, p.lat1, n[0], f[0], fluid);
@@ -218,8 +219,8 @@ __device__ __forceinline__ void update_two_lattice_rows(const int xi[NY], const 
                         if (cxd(d) != 0 && !((lk[j] >> d) & 1u)) f[j][d] += p.shift_cx[d];
                 }
             }
-            if (is_outlet_row(xi[j], yi[j], p)) outlet_fill<PREC>(f[j], jy_prev_at(p, yi[j]), p);
-            const auto m = collide<PREC>(f[j], p);
+            if (is_outlet_row(xi[j], yi[j], p)) outlet_fill<PREC, !STEP>(f[j], jy_prev_at(p, yi[j]), p);
+            const auto m = collide<PREC, !STEP>(f[j], p);
             if constexpr (STEP) step_collided();
 #pragma unroll
             for (int d = 0; d < 9; ++d) st<PREC>(p.lat1, lidx<L>(n[j], d, p.N), d, f[j][d], p);
@@ -300,13 +301,13 @@ template <int PREC> __device__ __forceinline__ unsigned vec_pack(float lo, float
 }
 
 // The scalar gather of a vector-kernel node that is not interior fluid (edges, obstacles, outlet).
-template <int PREC>
+template <int PREC, bool BATCH = false>
 __device__ __forceinline__ void vec_edge_gather(float *f, int x, int y, uint16_t lk, const StepParams &p)
 {
     const unsigned long long n = (unsigned long long)x + (unsigned long long)y * p.P;
 #pragma unroll
     for (int d = 0; d < 9; ++d) f[d] = pull_one<PREC, STREAM>(p.lat0, n, x, y, d, lk, p);
-    if (is_outlet_row(x, y, p)) outlet_fill<PREC>(f, jy_prev_at(p, y), p);
+    if (is_outlet_row(x, y, p)) outlet_fill<PREC, BATCH>(f, jy_prev_at(p, y), p);
 }
 
 template <int PREC>
