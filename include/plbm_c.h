@@ -264,8 +264,9 @@ int plbm_porous_disks(unsigned inner_w, unsigned inner_h, uint64_t seed, double 
 
 /* ---- batches of independent domains (no counterpart in the reference) ------------------
  * Many channels of different sizes, relaxation times and inlet densities advanced together:
- * PLBM_BATCH_PERSISTENT runs one persistent launch per step whose blocks take tiles of every
- * domain from a shared work queue; PLBM_BATCH_PERSISTENT_GRAPH replays runs of those steps from a
+ * PLBM_BATCH_PERSISTENT advances all domains in one launch, two plain steps at a time, and runs
+ * remaining and result steps as persistent launches whose blocks take tiles of every domain from a
+ * shared work queue; PLBM_BATCH_PERSISTENT_GRAPH replays runs of those steps from a
  * captured CUDA graph; PLBM_BATCH_PER_DOMAIN launches one kernel per domain per step (the
  * comparison).  Each domain is a channel with its own W x H mask (0 fluid, 1 solid; copied),
  * zero inlet/outlet velocity; nptl update, stream layout.  Precisions: PLBM_F32, PLBM_F16S,

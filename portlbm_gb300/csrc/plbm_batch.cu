@@ -1,6 +1,7 @@
-// plbm_batch.cu — many independent domains advanced together: one persistent launch per timestep
-// walks a queue of tiles drawn from every domain (atomic ticket counter, reset by a memset node),
-// and runs of steps are replayed from a captured CUDA graph.  Each domain keeps its own two
+// plbm_batch.cu — many independent domains advanced together: plain steps two a launch over pieces of
+// every domain (k_batch_two_steps); a step that writes results, or is left over, as one persistent
+// launch that walks a queue of tiles drawn from every domain (atomic ticket counter, reset by a
+// memset node).  Runs of steps are replayed from a captured CUDA graph.  Each domain keeps its own two
 // lattices (stream layout), links, geometry, relaxation time and boundary densities; the per-node
 // update is the nptl update of plbm_kernels.cuh (FP32, FP16 or BF16 shifted storage, or F64_Q60;
 // the 2-byte forms can run the vectorised row update, one warp per 256 consecutive nodes).
@@ -10,6 +11,7 @@
 #include "plbm_consts.h"
 #include "plbm_kernels.cuh"
 #include "plbm_launch.h"
+#include "plbm_pair.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -267,6 +269,30 @@ __global__ void __launch_bounds__(256, 2) k_batch_vec(BatchArgs a)
     }
 }
 
+// Two steps of every domain in one launch (plbm_pair.cuh).  A block's four warps take consecutive
+// (strip, rows) pieces of one domain; the hardware's block scheduler is the queue.  The domain's
+// parameters are staged in shared memory; 64 registers for FP32 (20 domains, 74.8 us a step; with 48,
+// 78.8), 48 for 2-byte storage (f16s 70.0; with 64, 73.3).
+struct BatchPairArgs {
+    const StepParams *params;      // two per domain: parity 0 and 1
+    const unsigned *block_domain;  // domain of each block
+    const unsigned *block_first;   // its first piece
+    int rows;                      // rows of a piece
+    unsigned parity;
+};
+template <int PREC>
+__global__ void __launch_bounds__(32 * PAIR_WARPS, PREC == F64_Q60 ? 5 : PREC == F32 ? 8 : 10) k_batch_two_steps(BatchPairArgs a)
+{
+    __shared__ __align__(16) StepParams sp;
+    const unsigned dom = a.block_domain[blockIdx.x];
+    const int piece = (int)a.block_first[blockIdx.x] + threadIdx.y;
+    stage_params(sp, a.params[2 * dom + a.parity]);
+    __syncthreads();
+    const int strips = (sp.W + PAIR_COLUMNS - 1) / PAIR_COLUMNS;
+    const int ya = piece / strips * a.rows;
+    if (ya < sp.H) march_two_steps<PREC, STREAM, false>(sp, piece % strips, ya, min(ya + a.rows, sp.H));   // warp-uniform
+}
+
 // One launch per domain with the same per-node update (the comparison the batching form is
 // measured against).
 template <int PREC>
@@ -305,6 +331,9 @@ struct plbm_batch {
     cudaStream_t stream = nullptr;
     cudaGraphExec_t gexec = nullptr;
     unsigned graph_steps = 0;
+    int pair_rows = 0;             // rows of a two-step launch's pieces; 0: single steps only (offsets too wide)
+    unsigned pair_blocks = 0;
+    unsigned *pair_domain_d = nullptr, *pair_first_d = nullptr;
     std::string err;
     unsigned long long nodes = 0;
     std::vector<unsigned> tile_domain_host;
@@ -317,6 +346,8 @@ struct plbm_batch {
         if (tile_domain_d) cudaFree(tile_domain_d);
         if (tile_local_d) cudaFree(tile_local_d);
         if (tiles_x_d) cudaFree(tiles_x_d);
+        if (pair_domain_d) cudaFree(pair_domain_d);
+        if (pair_first_d) cudaFree(pair_first_d);
         if (ticket_d) cudaFree(ticket_d);
         if (status_pending) cudaFree(status_pending);
         if (stream) cudaStreamDestroy(stream);
@@ -396,6 +427,77 @@ struct plbm_batch {
         return cudaGetLastError();
     }
 
+    // Plain steps run two a launch: the pieces of every domain are warps of one grid, where k_batch's few
+    // tiles of many rows leave SMs idle in small batches and HBM bounds it in large ones.  us a step,
+    // single steps (the tile of generate_dataset, or vectorised rows) -> two-step launches: 1 domain of
+    // 65 x 65 f32 21 -> 3.2; 4 domains, 0.16 M nodes: f32 28 -> 5.5, f16s 18 -> 6.2; 9 domains, 1.4 M:
+    // f32 46 -> 19, f16s 29 -> 20, f64_q60 64 -> 48; 20 domains, 6.9 M: f32 135 -> 75, f16s 89 -> 70,
+    // f16c 128 -> 94, f64_q60 221 -> 193.  Rows of a piece: enough pieces for every SM against rows done
+    // twice (0.07 M nodes f32, 1 / 2 / 4 rows: 3.9 / 4.5 / 6.0; 0.16 M: 6.0 / 5.5 / 6.9; 1.4 M, 2 / 4 / 8:
+    // 22 / 19 / 21; 6.9 M, 4 / 8 / 16: 78 / 75 / 79).
+    cudaError_t build_pairs()
+    {
+        unsigned long long padded = 0, offsets = 0;
+        const size_t eb = prec == PLBM_F32 ? 4 : prec == PLBM_F64_Q60 ? 8 : 2;
+        for (unsigned i = 0; i < n_domains(); ++i) {
+            padded += host[2 * i].N;
+            offsets = std::max<unsigned long long>(offsets, 9ull * host[2 * i].N * (eb == 8 ? 1 : eb));
+        }
+        if (offsets >= (1ull << 32)) return cudaSuccess;   // the kernel's offsets have 32 bits
+        const int rows = padded < (1ull << 17) ? 1 : padded < (1ull << 18) ? 2 : padded < (1ull << 21) ? 4
+                         : padded < (1ull << 25) ? 8 : 16;
+        std::vector<unsigned> dom, first;
+        for (unsigned i = 0; i < n_domains(); ++i) {
+            const StepParams &d = host[2 * i];
+            const unsigned pieces = (unsigned)((d.W + plbm::PAIR_COLUMNS - 1) / plbm::PAIR_COLUMNS * ((d.H + rows - 1) / rows));
+            for (unsigned k = 0; k < pieces; k += plbm::PAIR_WARPS) { dom.push_back(i); first.push_back(k); }
+        }
+        cudaError_t e = cudaMalloc(&pair_domain_d, dom.size() * sizeof(unsigned));
+        if (e == cudaSuccess) e = cudaMalloc(&pair_first_d, dom.size() * sizeof(unsigned));
+        if (e == cudaSuccess) e = cudaMemcpyAsync(pair_domain_d, dom.data(), dom.size() * 4, cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(pair_first_d, first.data(), dom.size() * 4, cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) return e;
+        pair_blocks = (unsigned)dom.size();
+        pair_rows = rows;
+        return cudaSuccess;
+    }
+
+    // Two steps in one launch from the lattices of parity `parity`, without results.
+    cudaError_t launch_two_steps(unsigned parity)
+    {
+        const plbm::BatchPairArgs a{ dom_d, pair_domain_d, pair_first_d, pair_rows, parity };
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(pair_blocks);
+        cfg.blockDim = dim3(32, plbm::PAIR_WARPS);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        switch (prec) {
+        case PLBM_F32: return cudaLaunchKernelEx(&cfg, plbm::k_batch_two_steps<plbm::F32>, a);
+        case PLBM_F16S: return cudaLaunchKernelEx(&cfg, plbm::k_batch_two_steps<plbm::F16S>, a);
+        case PLBM_BF16S: return cudaLaunchKernelEx(&cfg, plbm::k_batch_two_steps<plbm::BF16S>, a);
+        case PLBM_F16C: return cudaLaunchKernelEx(&cfg, plbm::k_batch_two_steps<plbm::F16C>, a);
+        default: return cudaLaunchKernelEx(&cfg, plbm::k_batch_two_steps<plbm::F64_Q60>, a);
+        }
+    }
+
+    // n steps from step t without results: four at a time in two two-step launches (step t's state
+    // stays in the lattices of its parity), the rest one by one.
+    cudaError_t enqueue_plain(unsigned t, unsigned n)
+    {
+        cudaError_t e = cudaSuccess;
+        for (; pair_rows && n >= 4 && e == cudaSuccess; t += 4, n -= 4) {
+            e = launch_two_steps(t & 1u);
+            if (e == cudaSuccess) e = launch_two_steps((t & 1u) ^ 1u);
+        }
+        for (; n > 0 && e == cudaSuccess; ++t, --n) e = launch(t, 0);
+        return e;
+    }
+
     cudaError_t launch_per_domain(unsigned step, int write_results)
     {
         const plbm::BatchArgs a = args(step & 1u, write_results);
@@ -420,8 +522,7 @@ struct plbm_batch {
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
-        cudaError_t el = cudaSuccess;
-        for (unsigned k = 0; k < steps_per_graph && el == cudaSuccess; ++k) el = launch(k, 0);
+        const cudaError_t el = enqueue_plain(0, steps_per_graph);
         e = cudaStreamEndCapture(stream, &g);
         if (el != cudaSuccess) return el;
         if (e != cudaSuccess) return e;
@@ -537,6 +638,7 @@ int plbm_batch_create(unsigned n, const plbm_batch_domain *doms, int precision, 
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
     b->blocks = sms * 8;
     if (e == cudaSuccess) e = b->build_tiles();
+    if (e == cudaSuccess) e = b->build_pairs();
     if (e != cudaSuccess) return fail(e, "batch set-up");
     *out = b;
     return PLBM_OK;
@@ -582,6 +684,10 @@ int plbm_batch_run(plbm_batch *b, unsigned steps, int mode, double *ms_per_step)
             e = cudaGraphLaunch(b->gexec, b->stream);
             k += per_graph;
         }
+    }
+    if (mode != PLBM_BATCH_PER_DOMAIN && k + 1 < steps && e == cudaSuccess) {
+        e = b->enqueue_plain(b->t + k, steps - 1 - k);
+        k = steps - 1;
     }
     for (; k < steps && e == cudaSuccess; ++k) {
         const int last = k + 1 == steps;

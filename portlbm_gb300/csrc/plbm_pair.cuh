@@ -136,17 +136,16 @@ __device__ __forceinline__ void pair_gather(CT<PREC> g[9], unsigned at, int xi, 
     if (lk & LINK_EDGE) fill_ghosts<PREC>(g, xi, yi, p);
 }
 
-template <int PREC, int L>
-__global__ void __launch_bounds__(32 * PAIR_WARPS, PREC == F64_Q60 ? 5 : L == COLLISION ? 8 : 10) k_two_steps(StepParams p, int rows)
+// One warp's rows [ya, yb) of strip `strip` (at least one column of it in the domain).  BATCH: the
+// parameters lie in shared memory (see CoefficientsF).
+template <int PREC, int L, bool BATCH = false>
+__device__ __forceinline__ void march_two_steps(const StepParams &p, int strip, int ya, int yb)
 {
     constexpr unsigned ALL = 0xffffffffu;
     const int lane = threadIdx.x;
-    const int strip = blockIdx.x * PAIR_WARPS + threadIdx.y;
-    if (strip * PAIR_COLUMNS >= p.W) return;                       // warp-uniform
     const int xi = strip * PAIR_COLUMNS - 1 + lane;
     const bool inx = xi >= 0 && xi < p.W;
     const bool writes = inx && lane >= 1 && lane <= PAIR_COLUMNS;
-    const int ya = blockIdx.y * rows, yb = min(ya + rows, p.H);
     auto link = [&](int y) -> uint16_t {
         return inx && y >= 0 && y < p.H ? link_at(p, (unsigned)(xi + y * p.P)) : (uint16_t)0;
     };
@@ -167,8 +166,8 @@ __global__ void __launch_bounds__(32 * PAIR_WARPS, PREC == F64_Q60 ? 5 : L == CO
         J jya = 0;
         if (lk & LINK_FLUID) {
             pair_gather<PREC, L>(a, at, xi, r, lk, p);
-            if (is_outlet_row(xi, r, p)) outlet_fill<PREC>(a, jy_prev_at(p, r), p);
-            const auto m = collide<PREC>(a, p);
+            if (is_outlet_row(xi, r, p)) outlet_fill<PREC, BATCH>(a, jy_prev_at(p, r), p);
+            const auto m = collide<PREC, BATCH>(a, p);
 #pragma unroll
             for (int d = 0; d < 9; ++d) a[d] = stored_value<PREC>(a[d], p);
             if (PREC != F64_Q60 || xi == p.W - 2) jya = column_half_jy(m, p);
@@ -205,7 +204,7 @@ __global__ void __launch_bounds__(32 * PAIR_WARPS, PREC == F64_Q60 ? 5 : L == CO
                         }
                     }
                 }
-                const auto m = collide<PREC>(f, p);
+                const auto m = collide<PREC, BATCH>(f, p);
 #pragma unroll
                 for (int d = 0; d < 9; ++d) {
                     using T = typename Store<PREC>::T;
@@ -226,6 +225,18 @@ __global__ void __launch_bounds__(32 * PAIR_WARPS, PREC == F64_Q60 ? 5 : L == CO
         lk_prev = lk;
         jyb = jya;
     }
+}
+
+// Launch bounds (blocks an SM) of the two-step kernels.
+template <int PREC, int L> struct PairBlocks { static constexpr int value = PREC == F64_Q60 ? 5 : L == COLLISION ? 8 : 10; };
+
+template <int PREC, int L>
+__global__ void __launch_bounds__(32 * PAIR_WARPS, PairBlocks<PREC, L>::value) k_two_steps(StepParams p, int rows)
+{
+    const int strip = blockIdx.x * PAIR_WARPS + threadIdx.y;
+    if (strip * PAIR_COLUMNS >= p.W) return;   // warp-uniform
+    const int ya = blockIdx.y * rows;
+    march_two_steps<PREC, L>(p, strip, ya, min(ya + rows, p.H));
 }
 
 }  // namespace plbm
