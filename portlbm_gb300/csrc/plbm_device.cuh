@@ -477,15 +477,12 @@ __device__ __forceinline__ Moments collide_q60(long long f[9], const StepParams 
 // doubles), on the FP64 pipe otherwise.
 __device__ __forceinline__ MomentsS collide_strict(double f[9], double omega)
 {
-    const unsigned long long ob = (unsigned long long)__double_as_longlong(omega);
-    // omega * 2^-60 and -omega * 2^-8 by their exponents; an omega outside [2^-500, 2^500] goes the
-    // other way (tested on the exponent field: a comparison would be an FP64 instruction)
-    const bool plain_omega = (unsigned)(ob >> 52) - 523u <= 1000u;
-    const double om60 = __longlong_as_double((long long)(ob - (60ull << 52)));
-    const double omc = __longlong_as_double((long long)((ob - (8ull << 52)) ^ (1ull << 63)));
+    // omega in [2^-500, 2^500], tested on the exponent field: a comparison would be an FP64 instruction
+    const unsigned exponent = (unsigned)((unsigned long long)__double_as_longlong(omega) >> 52);
+    const bool plain_omega = exponent - 523u <= 1000u;
     double g[9];
     strict::Fixed m;
-    if (strict::fast_collide(f, g, om60, omc, m) && plain_omega) {
+    if (strict::fast_collide(f, g, omega, m) && plain_omega) {
 #pragma unroll
         for (int d = 0; d < 9; ++d) f[d] = g[d];
         return { m.rho, m.jx, m.jy, m.usq122, true };

@@ -15,7 +15,7 @@
 // Converting |j| with I2F.F64 instead of by hand: 16.2 k; 4.5 a and 1.5 u^2 as FP64 products: 17.7 k.
 //
 // Fixed point: X = x * 2^61 in an int64.
-//  * A double x in [2^-8, 1) is a multiple of 2^-60, so X is exact and even.
+//  * A double x in [2^-7, 2) is a multiple of 2^-59, so X is exact and a multiple of 4.
 //  * Sums of such numbers are exact; rounding to 53 bits clears at most the low 10 bits (values below
 //    4).  It is done by the FP32 adder (rne): the low 12 bits as a float, plus 2^(23+k), minus it
 //    again, rounds them to a multiple of 2^k, ties to even, two instructions on a pipe that is
@@ -24,8 +24,8 @@
 //    into bit 0 (sticky): the other addend is a multiple of 4, so the sum lies on the same side of
 //    every rounding boundary as the exact one as long as k >= 2, i.e. for sums of at least 2^-7.
 //
-// The fast path needs every population in [2^-8, 1), density and momentum in the range checked in
-// `fast_collide` and |f - feq| < 2^-8; it says whether they were, and the caller otherwise runs the
+// The fast path needs every population in [2^-7, 2), density and momentum in the range checked in
+// `fast_collide` and |f - feq| < 2^-7; it says whether they were, and the caller otherwise runs the
 // plain FP64 sequence.  The code is shared with the host so that it can be compared with plain
 // double arithmetic there.
 #pragma once
@@ -150,13 +150,13 @@ PLBM_HD i64 rne_signed(i64 x)
     return (i64)round_low((u64)x, (uint32_t)e << 23);
 }
 
-// A population: exact for a double in [2^-8, 1); `bad` collects what is outside that range.
+// A population: exact for a double in [2^-7, 2); `bad` collects what is outside that range.
 PLBM_HD u64 to_fixed(double f, uint32_t &bad)
 {
     const u64 b = bits_of(f);
-    const uint32_t t = hi32(b) - (1015u << 20);      // exponent field 1015 .. 1022, sign 0
+    const uint32_t t = hi32(b) - (1016u << 20);      // exponent field 1016 .. 1023, sign 0
     bad |= t;                                        // any bit from 23 up: outside
-    const int sh = (int)((t >> 20) & 7u) + 1;
+    const int sh = (int)((t >> 20) & 7u) + 2;
     return join((hi32(b) & 0xFFFFFu) | 0x100000u, lo32(b)) << sh;
 }
 
@@ -217,9 +217,9 @@ PLBM_HD double magnitude(i64 x)
 
 struct Fixed { i64 rho, jx, jy; double usq122; };   // moments: x * 2^61, and u^2 * 2^122
 
-// The BGK update of collide_f64_strict for omega > 0 (om60 = omega * 2^-60, omc = -omega * 2^-8).
+// The BGK update of collide_f64_strict for omega in [2^-500, 2^500].
 // True when every value was in range; f then holds the new populations (f_out) and `m` the moments.
-PLBM_HD bool fast_collide(const double f[9], double f_out[9], double om60, double omc, Fixed &m)
+PLBM_HD bool fast_collide(const double f[9], double f_out[9], double omega, Fixed &m)
 {
     uint32_t bad = 0;
     u64 F[9];
@@ -262,18 +262,22 @@ PLBM_HD bool fast_collide(const double f[9], double f_out[9], double om60, doubl
         feq[dp] = weigh(up, k < 2 ? w9h : w36h, k < 2 ? w9l : w36l);
         feq[8 - dp] = weigh(dn, k < 2 ? w9h : w36h, k < 2 ? w9l : w36l);
     }
+    // -omega (f - feq): the difference is exact, a multiple of 2^-59 (both are at least 2^-7), and below
+    // 2^-7 its magnitude is the mantissa of 2^52 + |D|; the fused multiply-add of that rounds omega * |D|
+    // once.  (An inlet 0.2 denser than the channel keeps its column just below that: with 2^-8 the column's
+    // warps took both paths and a step of the 400 x 100 channel 8.2 us instead of 6.4.)
+    const u64 ob = bits_of(omega);
+    const double om = from_bits(ob - (59ull << 52)), omc = from_bits((ob - (7ull << 52)) ^ (1ull << 63));
     uint32_t far = 0;
 #if defined(__CUDACC__)
 #pragma unroll
 #endif
     for (int d = 0; d < 9; ++d) {
-        // -omega (f - feq): f - feq is exact (a multiple of 2^-60), and below 2^-8 its magnitude is the
-        // mantissa of 2^52 + |D|; the fused multiply-add of it rounds omega * |D| once
-        const i64 D = (i64)(F[d] - feq[d]) >> 1;                     // units of 2^-60
+        const i64 D = (i64)(F[d] - feq[d]) >> 2;                     // units of 2^-59
         const uint32_t s = (uint32_t)((int32_t)hi32((u64)D) >> 31);
         const u64 mag = ((u64)D ^ join(s, s)) - join(s, s);
         far |= hi32(mag);
-        const double P = fma_rn(om60, from_bits(mag | 0x4330000000000000ull), omc);
+        const double P = fma_rn(om, from_bits(mag | 0x4330000000000000ull), omc);
         const u64 pb = bits_of(P);
         f_out[d] = plus_rn(from_bits(join(hi32(pb) ^ (~s & 0x80000000u), lo32(pb))), f[d]);
     }

@@ -61,7 +61,7 @@ int main(int argc, char **argv)
         const double omega = 1 / (0.5 + u(g));
         plain(r, omega, m);
         Fixed x;
-        if (!fast_collide(f, o, omega * 0x1p-60, -omega * 0x1p-8, x)) continue;
+        if (!fast_collide(f, o, omega, x)) continue;
         ++compared;
         bool same = (double)x.rho * 0x1p-61 == m[0] && (double)x.jx * 0x1p-61 == m[1] && (double)x.jy * 0x1p-61 == m[2] &&
                     x.usq122 * 0x1p-122 == m[3];
