@@ -7,6 +7,7 @@
 //
 // No counterpart in the reference: this is the learned warm-start addition of the GB300 build.
 #include "../../include/plbm_c.h"
+#include "plbm_nn_launch.cuh"
 
 #include <cuda_bf16.h>
 #include <mutex>
@@ -324,6 +325,7 @@ __global__ void k_adam_dev(float *w, const float *g, float *m, float *v, __nv_bf
 // features[n][0..2] as constant planes; channels beyond 4 are zero.
 __global__ void k_assemble(const int8_t *mask, const float *features, __nv_bfloat16 *y, int N, int H, int W, int C)
 {
+    nn_begin();
     const long long total = (long long)N * H * W;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < total; p += (long long)gridDim.x * blockDim.x) {
         const int n = (int)(p / ((long long)H * W));
@@ -421,6 +423,7 @@ __global__ void k_relu_bwd_v(const uint4 *y, uint4 *g, unsigned n8)
 
 __global__ void k_add_v(const uint4 *a, const uint4 *b, uint4 *y, unsigned n8)
 {
+    nn_begin();
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += gridDim.x * blockDim.x) {
         float fa[8], fb[8];
         unpack8(a[i], fa);
@@ -434,6 +437,7 @@ __global__ void k_add_v(const uint4 *a, const uint4 *b, uint4 *y, unsigned n8)
 // Output unit i of [N][H][W][CU] (H, W the output size) from input unit (n, yy / 2, xx / 2).
 __global__ void k_up2_v(const uint4 *x, uint4 *y, unsigned N, unsigned H, unsigned W, unsigned CU)
 {
+    nn_begin();
     const unsigned total = N * H * W * CU;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const unsigned cu = i % CU, t = i / CU, xx = t % W, t2 = t / W, yy = t2 % H, n = t2 / H;
@@ -466,6 +470,7 @@ __global__ void k_up2_bwd_v(const uint4 *gy, uint4 *gx, unsigned N, unsigned H, 
 // Output unit i of [N][H/2][W/2][CU] (H, W the input size): the mean of its four input units.
 __global__ void k_pool2_v(const uint4 *x, uint4 *y, unsigned N, unsigned H, unsigned W, unsigned CU)
 {
+    nn_begin();
     const unsigned Ho = H / 2, Wo = W / 2, total = N * Ho * Wo * CU;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const unsigned cu = i % CU, t = i / CU, xo = t % Wo, t2 = t / Wo, yo = t2 % Ho, n = t2 / Ho;
@@ -499,6 +504,7 @@ __global__ void k_pool2_bwd_v(const uint4 *gy, uint4 *gx, unsigned N, unsigned H
     }
 }
 
+int launched(cudaError_t e) { return e == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA; }
 int grid_for(long long n) { return (int)((n + 255) / 256 < 152 * 16 ? (n + 255) / 256 : 152 * 16); }
 
 // The 16-byte forms apply: C a multiple of 8, every pointer 16-byte aligned, units below 2^31.
@@ -657,9 +663,8 @@ int plbm_nn_relu_bwd(const void *y, void *g, long long n, void *stream)
 int plbm_nn_pool2(const void *x, void *y, int N, int H, int W, int C, void *stream)
 {
     if (vec8(C, (long long)N * H * W * C, x, y)) {
-        k_pool2_v<<<grid_for((long long)N * H * W * C / 32), 256, 0, (cudaStream_t)stream>>>(
-            (const uint4 *)x, (uint4 *)y, N, H, W, C / 8);
-        return cudaGetLastError() == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
+        return launched(nn_launch(k_pool2_v, (unsigned)grid_for((long long)N * H * W * C / 32), 256, 0, (cudaStream_t)stream,
+                                  (const uint4 *)x, (uint4 *)y, N, H, W, C / 8));
     }
     k_pool2<<<grid_for((long long)N * H * W * C / 4), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)x,
                                                                                        (__nv_bfloat16 *)y, N, H, W, C);
@@ -681,9 +686,8 @@ int plbm_nn_pool2_bwd(const void *gy, void *gx, int N, int H, int W, int C, void
 int plbm_nn_up2(const void *x, void *y, int N, int H, int W, int C, void *stream)
 {
     if (vec8(C, (long long)N * H * W * C, x, y)) {
-        k_up2_v<<<grid_for((long long)N * H * W * C / 8), 256, 0, (cudaStream_t)stream>>>(
-            (const uint4 *)x, (uint4 *)y, N, H, W, C / 8);
-        return cudaGetLastError() == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
+        return launched(nn_launch(k_up2_v, (unsigned)grid_for((long long)N * H * W * C / 8), 256, 0, (cudaStream_t)stream,
+                                  (const uint4 *)x, (uint4 *)y, N, H, W, C / 8));
     }
     k_up2<<<grid_for((long long)N * H * W * C), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)x,
                                                                                  (__nv_bfloat16 *)y, N, H, W, C);
@@ -705,9 +709,8 @@ int plbm_nn_up2_bwd(const void *gy, void *gx, int N, int H, int W, int C, void *
 int plbm_nn_add(const void *a, const void *b, void *y, long long n, void *stream)
 {
     if (vec8(8, n, a, b, y)) {
-        k_add_v<<<grid_for(n / 8), 256, 0, (cudaStream_t)stream>>>((const uint4 *)a, (const uint4 *)b, (uint4 *)y,
-                                                                  (unsigned)(n / 8));
-        return cudaGetLastError() == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
+        return launched(nn_launch(k_add_v, (unsigned)grid_for(n / 8), 256, 0, (cudaStream_t)stream, (const uint4 *)a,
+                                  (const uint4 *)b, (uint4 *)y, (unsigned)(n / 8)));
     }
     k_add<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)a, (const __nv_bfloat16 *)b,
                                                          (__nv_bfloat16 *)y, n);
@@ -742,9 +745,8 @@ int plbm_nn_adam_dev(float *w, const float *g, float *m, float *v, void *wb, lon
 int plbm_nn_assemble(const int8_t *mask, const float *features, void *y, int N, int H, int W, int C, void *stream)
 {
     if (N <= 0 || H <= 0 || W <= 0 || C < 4) return PLBM_ERR_ARGUMENT;
-    k_assemble<<<grid_for((long long)N * H * W), 256, 0, (cudaStream_t)stream>>>(mask, features, (__nv_bfloat16 *)y,
-                                                                                 N, H, W, C);
-    return cudaGetLastError() == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
+    return launched(nn_launch(k_assemble, (unsigned)grid_for((long long)N * H * W), 256, 0, (cudaStream_t)stream, mask, features,
+                              (__nv_bfloat16 *)y, N, H, W, C));
 }
 
 }  // extern "C"

@@ -15,6 +15,7 @@
 // Every wait is bounded (about 1 s): on expiry the thread records an error in g_tc_error, stops
 // its role, waits (bounded) for its own copies in flight, the CTA frees its TMEM and returns.
 #include "../../include/plbm_c.h"
+#include "plbm_nn_launch.cuh"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -29,10 +30,10 @@ namespace {
 
 constexpr int TC_BM = 128;          // output pixels per CTA (TMEM lanes)
 constexpr int TC_KB = 32;           // channels per K block (64-byte rows)
-constexpr int TC_STAGES = 4;
+constexpr int TC_STAGES = 4, TC_MAX_STAGES = 12;
 constexpr int TC_A_BYTES = TC_BM * TC_KB * 2;        // 8 KB
 constexpr int TC_B_MAX = 128 * TC_KB * 2;            // 8 KB at Npad = 128
-constexpr int TC_SMEM = TC_STAGES * (TC_A_BYTES + TC_B_MAX) + 1024 /* alignment */ + 256 /* barriers */;   // largest
+constexpr int TC_SMEM = TC_MAX_STAGES * (TC_A_BYTES + TC_B_MAX) + 1024 /* alignment */ + 256 /* barriers */;   // largest
 constexpr long long TC_WAIT_CYCLES = 2000000000ll;   // ~1 s at the maximum SM clock
 
 __device__ int g_tc_error;
@@ -145,6 +146,7 @@ struct TcArgs {
     int N, H, W, Cin, Cout, npad, relu;
     int BW, BH, tiles_x, tiles_y;
     int stage_bytes;        // A tile + the B tile rounded up to 1024 B
+    int stages;
     int *err;
 };
 
@@ -155,15 +157,15 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
     // stages aligned to 1024 B (the swizzle pattern repeats every 512 B)
     unsigned char *smem = tc_smem_raw + ((1024 - (smem_u32(tc_smem_raw) & 1023)) & 1023);
-    unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem + TC_STAGES * a.stage_bytes);
-    unsigned long long *full = bars, *empty = bars + TC_STAGES, *done = bars + 2 * TC_STAGES;
-    unsigned *tmem_slot = reinterpret_cast<unsigned *>(bars + 2 * TC_STAGES + 1);
+    unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem + a.stages * a.stage_bytes);
+    unsigned long long *full = bars, *empty = bars + a.stages, *done = bars + 2 * a.stages;
+    unsigned *tmem_slot = reinterpret_cast<unsigned *>(bars + 2 * a.stages + 1);
     int *counts = reinterpret_cast<int *>(tmem_slot + 1);   // [0] issued, [1] consumed, [2] failed
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned ncols = a.npad <= 32 ? 32u : (a.npad <= 64 ? 64u : 128u);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < TC_STAGES; ++s) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
+        for (int s = 0; s < a.stages; ++s) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
         mbar_init(smem_u32(done), 1);
         counts[0] = counts[1] = counts[2] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -173,6 +175,7 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
                      "r"(ncols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    nn_begin();
     stage_bias(s_bias, a.bias, a.Cout, a.npad);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -188,9 +191,8 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
     const unsigned bbytes = (unsigned)a.npad * TC_KB * 2;
 
     if (warp == 0 && lane == 0) {              // producer: TMA loads
-        for (int it = 0; it < iters; ++it) {
-            const int s = it % TC_STAGES;
-            if (it >= TC_STAGES && !mbar_wait(smem_u32(&empty[s]), (unsigned)((it / TC_STAGES - 1) & 1))) {
+        for (int it = 0, s = 0, round = 0; it < iters; ++it, s = s + 1 == a.stages ? (++round, 0) : s + 1) {
+            if (round > 0 && !mbar_wait(smem_u32(&empty[s]), (unsigned)((round - 1) & 1))) {
                 counts[2] = 1;
                 break;
             }
@@ -205,10 +207,8 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
         }
     } else if (warp == 1 && lane == 0) {       // MMA issuer
         const unsigned idesc = instr_desc(a.npad);
-        int it = 0;
-        for (; it < iters; ++it) {
-            const int s = it % TC_STAGES;
-            if (!mbar_wait(smem_u32(&full[s]), (unsigned)((it / TC_STAGES) & 1))) {
+        for (int it = 0, s = 0, round = 0; it < iters; ++it, s = s + 1 == a.stages ? (++round, 0) : s + 1) {
+            if (!mbar_wait(smem_u32(&full[s]), (unsigned)(round & 1))) {
                 counts[2] = 1;
                 break;
             }
@@ -249,7 +249,7 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
         // flight (their stages' full barriers), each bounded, before the TMEM is released
         mbar_wait(smem_u32(done), 0);
         for (int it = counts[1]; it < counts[0]; ++it)
-            mbar_wait(smem_u32(&full[it % TC_STAGES]), (unsigned)((it / TC_STAGES) & 1));
+            mbar_wait(smem_u32(&full[it % a.stages]), (unsigned)((it / a.stages) & 1));
     }
     __syncthreads();
     if (warp == 0) {
@@ -770,6 +770,7 @@ __global__ void __launch_bounds__(SM_BUILD, 8) k_conv_small_tc(SmallArgs a)
                      "r"(ncols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    nn_begin();
     stage_bias(s_bias, a.bias, a.Cout, a.npad);
     const int per_img = a.tiles_x * a.tiles_y;
     const int n = blockIdx.x / per_img, t2 = blockIdx.x % per_img;
@@ -1031,6 +1032,7 @@ k_conv_halo_tc(const __grid_constant__ CUtensorMap hmap, const __grid_constant__
                      "r"(ncols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    nn_begin();
     stage_bias(s_bias, a.bias, a.Cout, a.npad);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -1274,15 +1276,20 @@ int plbm_nn_tc_conv(const void *x, const void *w, const float *bias, void *y, in
         }
         HaloArgs h{ (__nv_bfloat16 *)y, bias, N, H, W, Cin, Cout, npad, relu, W / TC_BM, N * H * (W / TC_BM),
                     kblocks, hstages, w_bytes, err };
-        k_conv_halo_tc<<<h.tiles < sms ? h.tiles : sms, 224, smem, s>>>(hmap, wmap, h);
-        return cudaGetLastError() == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
+        return nn_launch(k_conv_halo_tc, (unsigned)(h.tiles < sms ? h.tiles : sms), 224, smem, s, hmap, wmap, h) == cudaSuccess
+                   ? PLBM_OK : PLBM_ERR_CUDA;
     }
     // stages sized by the padded output channels, so narrow layers fit more CTAs per SM
     const int stage = TC_A_BYTES + (npad * TC_KB * 2 + 1023) / 1024 * 1024;
-    TcArgs a{ (__nv_bfloat16 *)y, bias, N, H, W, Cin, Cout, npad, relu, BW, BH, W / BW, H / BH, stage, err };
-    const int tiles = N * a.tiles_x * a.tiles_y;
-    k_conv_tc<<<tiles, 128, TC_STAGES * stage + 1024 + 256, s>>>(xmap, wmap, a);
-    return cudaGetLastError() == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
+    const int tiles = N * (W / BW) * (H / BH);
+    // four stages let four CTAs share an SM; a layer with fewer tiles than SMs waits for its own loads
+    // instead and takes all that fit (16 x 16 pixels, 128 -> 128 channels: 36 stages' worth of loads; a
+    // 1 x 256^2 inference 215 -> 210 us, a 5 x 256^2 one 318 -> 309)
+    const int fit = (TC_SMEM - 1024 - 256) / stage, most = fit < TC_MAX_STAGES ? fit : TC_MAX_STAGES;
+    const int stages = tiles <= sms ? most : tiles <= 2 * sms ? (most + 1) / 2 : TC_STAGES;
+    TcArgs a{ (__nv_bfloat16 *)y, bias, N, H, W, Cin, Cout, npad, relu, BW, BH, W / BW, H / BH, stage, stages, err };
+    return nn_launch(k_conv_tc, (unsigned)tiles, 128, (size_t)stages * stage + 1024 + 256, s, xmap, wmap, a) == cudaSuccess
+               ? PLBM_OK : PLBM_ERR_CUDA;
 }
 
 // The weight gradient runs on the TMA-fed tensor-core kernel for Cin a multiple of 32 up to 128,
@@ -1431,8 +1438,8 @@ int plbm_nn_tc_small_conv(const void *x, const void *w, const float *bias, void 
     a.kchunks = (9 * Cin + TC_KB - 1) / TC_KB;
     a.err = err;
     const int smem = a.kchunks * (WG_CHUNK + a.npad * 64) + 1024 + 64;
-    k_conv_small_tc<<<N * a.tiles_x * a.tiles_y, SM_BUILD, smem, s>>>(a);
-    return cudaGetLastError() == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
+    return nn_launch(k_conv_small_tc, (unsigned)(N * a.tiles_x * a.tiles_y), SM_BUILD, smem, s, a) == cudaSuccess ? PLBM_OK
+                                                                                                                : PLBM_ERR_CUDA;
 }
 
 // Weight gradient of a layer with Cin <= 32 (its 9 * Cin (tap, ci) columns in at most 9 chunks of 32)
