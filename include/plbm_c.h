@@ -327,6 +327,21 @@ int plbm_nn_pool2_bwd(const void *gy, void *gx, int N, int H, int W, int C, void
 int plbm_nn_up2(const void *x, void *y, int N, int H, int W, int C, void *stream);
 int plbm_nn_up2_bwd(const void *gy, void *gx, int N, int H, int W, int C, void *stream);
 int plbm_nn_add(const void *a, const void *b, void *y, long long n, void *stream);
+/* plbm_nn_assemble for four channels with the scalars on the host (3 N floats, read during the call):
+ * no copy and no synchronisation.  y 8-byte aligned. */
+int plbm_nn_assemble_host(const int8_t *mask, const float *features, void *y, int N, int H, int W, void *stream);
+/* The operator's whole forward pass in one call: per level two convolutions and, but for the last, a
+ * 2x2 average pooling; back up per level nearest upsampling, a convolution, the skip addition of the
+ * level's encoder output and a convolution; the head.  layers: 2 levels + 2 (levels - 1) + 1 of them in
+ * that order.  acts: the device buffers the results go to, in the order they are computed (each layer's,
+ * pooling's, upsampling's and addition's). */
+typedef struct {
+    const void *w;
+    const float *bias;
+    int cin, cout, relu;
+} plbm_nn_layer;
+int plbm_nn_unet_forward(const void *x, void *const *acts, const plbm_nn_layer *layers, int levels, int N, int H, int W,
+                         void *stream);
 int plbm_nn_mse(const void *pred, const float *target, const int8_t *mask, void *grad, float *loss, long long P, int C,
                 float inv_count, void *stream);
 int plbm_nn_adam(float *w, const float *g, float *m, float *v, void *w_bf16, long long n, float lr, float b1, float b2,

@@ -334,6 +334,22 @@ __global__ void k_assemble(const int8_t *mask, const float *features, __nv_bfloa
     }
 }
 
+// The same for four channels and up to ASSEMBLE_SAMPLES samples whose scalars come with the launch.
+constexpr int ASSEMBLE_SAMPLES = 64;
+struct AssembleValues { float v[ASSEMBLE_SAMPLES][3]; };
+__global__ void k_assemble_values(const int8_t *mask, AssembleValues a, uint2 *y, int N, unsigned pixels)
+{
+    nn_begin();
+    for (unsigned n = blockIdx.y; n < (unsigned)N; n += gridDim.y) {
+        const __nv_bfloat162 b = __floats2bfloat162_rn(a.v[n][1], a.v[n][2]);
+        for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < pixels; p += gridDim.x * blockDim.x) {
+            const size_t i = (size_t)n * pixels + p;
+            const __nv_bfloat162 m = __floats2bfloat162_rn((float)mask[i], a.v[n][0]);
+            y[i] = make_uint2(*reinterpret_cast<const unsigned *>(&m), *reinterpret_cast<const unsigned *>(&b));
+        }
+    }
+}
+
 // ---- 16-byte forms: eight channels per thread and 32-bit index arithmetic, for channel counts that
 // are multiples of 8 (every layer of the operator but its 4-channel input and 3-channel output) ----
 __device__ __forceinline__ void unpack8(const uint4 u, float f[8])
@@ -715,6 +731,76 @@ int plbm_nn_add(const void *a, const void *b, void *y, long long n, void *stream
     k_add<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)a, (const __nv_bfloat16 *)b,
                                                          (__nv_bfloat16 *)y, n);
     return cudaGetLastError() == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
+}
+
+int plbm_nn_assemble_host(const int8_t *mask, const float *features, void *y, int N, int H, int W, void *stream)
+{
+    if (!mask || !features || !y || N < 0 || H < 1 || W < 1 || (long long)H * W > 0x7fffffffll) return PLBM_ERR_ARGUMENT;
+    const size_t pixels = (size_t)H * W;
+    for (int n0 = 0; n0 < N; n0 += ASSEMBLE_SAMPLES) {
+        const int n = N - n0 < ASSEMBLE_SAMPLES ? N - n0 : ASSEMBLE_SAMPLES;
+        AssembleValues a{};
+        for (int i = 0; i < 3 * n; ++i) a.v[i / 3][i % 3] = features[3 * n0 + i];
+        cudaLaunchConfig_t cfg{};
+        const unsigned blocks = (unsigned)((pixels + 255) / 256);
+        cfg.gridDim = dim3(blocks < 256 ? blocks : 256, (unsigned)n);
+        cfg.blockDim = dim3(256);
+        cfg.stream = (cudaStream_t)stream;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_assemble_values, mask + n0 * pixels, a,
+                                                 (uint2 *)((__nv_bfloat16 *)y + 4 * n0 * pixels), n, (unsigned)pixels);
+        if (e != cudaSuccess) return PLBM_ERR_CUDA;
+    }
+    return PLBM_OK;
+}
+
+int plbm_nn_unet_forward(const void *x, void *const *acts, const plbm_nn_layer *layers, int levels, int N, int H, int W,
+                         void *stream)
+{
+    if (!x || !acts || !layers || levels < 1) return PLBM_ERR_ARGUMENT;
+    const plbm_nn_layer *layer = layers;
+    void *const *next = acts;
+    int rc = PLBM_OK;
+    auto conv = [&](const void *in, int h, int w) -> void * {
+        void *y = *next++;
+        if (rc == PLBM_OK)
+            rc = plbm_nn_conv_fwd(in, layer->w, layer->bias, y, N, h, w, layer->cin, layer->cout, layer->relu, stream);
+        ++layer;
+        return y;
+    };
+    const void *skip[32] = {};
+    int width[32] = {};
+    if (levels > 32) return PLBM_ERR_ARGUMENT;
+    const void *cur = x;
+    for (int l = 0; l < levels; ++l) {
+        const int h = H >> l, w = W >> l;
+        cur = conv(cur, h, w);
+        cur = conv(cur, h, w);
+        skip[l] = cur;
+        width[l] = layer[-1].cout;
+        if (l + 1 < levels) {
+            void *p = *next++;
+            if (rc == PLBM_OK) rc = plbm_nn_pool2(cur, p, N, h, w, width[l], stream);
+            cur = p;
+        }
+    }
+    int c = width[levels - 1];
+    for (int l = levels - 2; l >= 0; --l) {
+        const int h = H >> l, w = W >> l;
+        void *u = *next++;
+        if (rc == PLBM_OK) rc = plbm_nn_up2(cur, u, N, h, w, c, stream);
+        const void *a = conv(u, h, w);
+        c = layer[-1].cout;
+        void *sum = *next++;
+        if (rc == PLBM_OK) rc = plbm_nn_add(a, skip[l], sum, (long long)N * h * w * c, stream);
+        cur = conv(sum, h, w);
+    }
+    conv(cur, H, W);
+    return rc;
 }
 
 int plbm_nn_mse(const void *pred, const float *target, const int8_t *mask, void *grad, float *loss, long long P, int C,

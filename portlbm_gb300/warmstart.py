@@ -30,6 +30,8 @@ csrc/plbm_batch.cu), see `generate_dataset`.
 from __future__ import annotations
 
 import ctypes
+import functools
+import math
 import time
 
 import numpy as np
@@ -60,6 +62,8 @@ def _fns():
         "plbm_nn_up2_bwd": [vp, vp, i, i, i, i, vp],
         "plbm_nn_add": [vp, vp, vp, ll, vp],
         "plbm_nn_mse": [vp, vp, vp, vp, vp, ll, i, f, vp],
+        "plbm_nn_assemble_host": [vp, vp, vp, i, i, i, vp],
+        "plbm_nn_unet_forward": [vp, vp, vp, i, i, i, i, vp],
         "plbm_nn_adam": [vp, vp, vp, vp, vp, ll, f, f, f, f, i, vp],
         "plbm_nn_adam_dev": [vp, vp, vp, vp, vp, ll, vp, f, f, f, vp, vp],
         "plbm_nn_assemble": [vp, vp, vp, i, i, i, i, vp],
@@ -152,6 +156,53 @@ class Params:
         return tuple(t[a:a + n].view(shape) for t in (self.w, self.g, self.m, self.v, self.wb, self.wbt))
 
 
+LEVELS = len(WIDTHS)
+
+
+class _CLayer(ctypes.Structure):
+    _fields_ = [("w", ctypes.c_void_p), ("bias", ctypes.c_void_p), ("cin", ctypes.c_int), ("cout", ctypes.c_int),
+                ("relu", ctypes.c_int)]
+
+
+@functools.lru_cache(maxsize=32)
+def forward_plan(n, h, w):
+    """The forward pass's activations in the order plbm_nn_unet_forward writes them, but for the
+    prediction: ((name, element offset, shape), ...) and the buffer's elements.  Every piece starts on
+    256 bytes."""
+    plan, at = [], 0
+
+    def add(name, lvl, c):
+        nonlocal at
+        shape = (n, h >> lvl, w >> lvl, c)
+        plan.append((name, at, shape))
+        at += -(-math.prod(shape) // PARAM_ALIGN) * PARAM_ALIGN
+
+    for lvl in range(LEVELS):
+        add(f"e{lvl}a", lvl, WIDTHS[lvl])
+        add(f"e{lvl}b", lvl, WIDTHS[lvl])
+        if lvl < LEVELS - 1:
+            add(f"p{lvl}", lvl + 1, WIDTHS[lvl])
+    for k, lvl in enumerate(range(LEVELS - 2, -1, -1)):
+        add(f"u{lvl}", lvl, DEC[2 * k][0])
+        for name in (f"d{lvl}a", f"s{lvl}", f"d{lvl}b"):
+            add(name, lvl, DEC[2 * k][1])
+    return tuple(plan), at
+
+
+class Activations:
+    """The tensors of a forward pass by name ("in", "e0a", ..., "out"), made from its buffer when asked for."""
+
+    def __init__(self, x, work, plan, out):
+        self._work, self._plan = work, {name: (off, shape) for name, off, shape in plan}
+        self._given = {"in": x, "out": out}
+
+    def __getitem__(self, name):
+        if name in self._given:
+            return self._given[name]
+        off, shape = self._plan[name]
+        return self._work[off:off + math.prod(shape)].view(shape)
+
+
 class NeuralOperator:
     """U-Net-style operator; forward/backward/Adam all run in libplbm's kernels."""
 
@@ -203,43 +254,22 @@ class NeuralOperator:
     def _buf(self, n, h, w, c):
         return self.torch.empty((n, h, w, c), dtype=self.torch.bfloat16, device="cuda")
 
-    def _conv(self, layer, x, n, h, w):
-        y = self._buf(n, h, w, layer.cout)
-        _ok(self.lib.plbm_nn_conv_fwd(x.data_ptr(), layer.wb.data_ptr(), layer.b.data_ptr(), y.data_ptr(), n, h, w,
-                                      layer.cin, layer.cout, int(layer.relu), self._s))
-        return y
-
     def forward(self, x, n, h, w):
-        """x: [n,h,w,4] bf16 input; returns the [n,h,w,3] prediction and keeps activations for backward."""
+        """x: [n,h,w,4] bf16 input; returns the [n,h,w,3] prediction and keeps activations for backward.
+
+        One native call launches every kernel (39 launches from Python took longer than they ran); the
+        activations are pieces of one buffer, the prediction a tensor of its own."""
         self._s = self._stream()
-        acts = {"in": x}
-        cur, hh, ww = x, h, w
-        skips = []
-        for lvl in range(5):
-            a = self._conv(self.enc[2 * lvl], cur, n, hh, ww)
-            b = self._conv(self.enc[2 * lvl + 1], a, n, hh, ww)
-            acts[f"e{lvl}a"], acts[f"e{lvl}b"] = a, b
-            skips.append((b, hh, ww))
-            if lvl < 4:
-                p = self._buf(n, hh // 2, ww // 2, b.shape[-1])
-                _ok(self.lib.plbm_nn_pool2(b.data_ptr(), p.data_ptr(), n, hh, ww, b.shape[-1], self._s))
-                acts[f"p{lvl}"] = p
-                cur, hh, ww = p, hh // 2, ww // 2
-            else:
-                cur = b
-        for k, lvl in enumerate((3, 2, 1, 0)):
-            sh, sw = skips[lvl][1], skips[lvl][2]
-            u = self._buf(n, sh, sw, cur.shape[-1])
-            _ok(self.lib.plbm_nn_up2(cur.data_ptr(), u.data_ptr(), n, sh, sw, cur.shape[-1], self._s))
-            a = self._conv(self.dec[2 * k], u, n, sh, sw)
-            s = self._buf(n, sh, sw, a.shape[-1])
-            _ok(self.lib.plbm_nn_add(a.data_ptr(), skips[lvl][0].data_ptr(), s.data_ptr(), s.numel(), self._s))
-            b = self._conv(self.dec[2 * k + 1], s, n, sh, sw)
-            acts[f"u{lvl}"], acts[f"d{lvl}a"], acts[f"s{lvl}"], acts[f"d{lvl}b"] = u, a, s, b
-            cur = b
-        out = self._conv(self.head, cur, n, h, w)
-        acts["out"] = out
-        self.acts, self.shape = acts, (n, h, w)
+        torch = self.torch
+        plan, total = forward_plan(n, h, w)
+        work = torch.empty(total, dtype=torch.bfloat16, device="cuda")
+        out = self._buf(n, h, w, self.head.cout)
+        base = work.data_ptr()
+        acts = (ctypes.c_void_p * (len(plan) + 1))(*[base + 2 * off for _, off, _ in plan], out.data_ptr())
+        layers = (_CLayer * len(self.layers))(*[_CLayer(l.wb.data_ptr(), l.b.data_ptr(), l.cin, l.cout, int(l.relu))
+                                                for l in self.layers])
+        _ok(self.lib.plbm_nn_unet_forward(x.data_ptr(), acts, layers, LEVELS, n, h, w, self._s))
+        self.acts, self.shape = Activations(x, work, plan, out), (n, h, w)
         return out
 
     def _conv_bwd(self, layer, x, y, gy, n, h, w, need_gx=True):
@@ -354,12 +384,11 @@ class NeuralOperator:
 
     def assemble(self, masks, feats):
         """masks: [n,h,w] int8 device tensor; feats: n rows of `features` -> [n,h,w,4] bf16 input."""
-        torch = self.torch
         n, h, w = masks.shape
         self._s = self._stream()
         x = self._buf(n, h, w, C_IN)
-        f = torch.tensor(np.asarray(feats, dtype=np.float32).reshape(n, 3), device="cuda")
-        _ok(self.lib.plbm_nn_assemble(masks.data_ptr(), f.data_ptr(), x.data_ptr(), n, h, w, C_IN, self._s))
+        f = np.ascontiguousarray(np.asarray(feats, dtype=np.float32).reshape(n, 3))
+        _ok(self.lib.plbm_nn_assemble_host(masks.data_ptr(), f.ctypes.data, x.data_ptr(), n, h, w, self._s))
         return x
 
     def predict(self, mask: np.ndarray, rin: float, rout: float, tau: float, sigma: float = 16.0):
