@@ -11,8 +11,9 @@ algorithm, stream layout.  A "step" is one lattice-Boltzmann timestep over the w
                  live: max |GPU - oracle| of rho, jx, jy after 2000 steps of the 400x100 channel.
 * ``e2e``        the same metric through the public API with host buffers: create_handler from
                  host properties + host mask (H2D), K steps, results read back (D2H), all timed.
-* ``roofline``   HBM roofline of the step kernel: 144 algorithmic bytes per node update (9 loads +
-                 9 stores of 8 B) / CUDA-event time per launch, against MEASURED_PEAKS.json.
+* ``roofline``   HBM roofline of the step kernels: 144 algorithmic bytes per node and launch (9 loads
+                 + 9 stores of 8 B; plain steps of large domains run two a launch, so they need these
+                 bytes once for two steps) x launches / CUDA-event time, against MEASURED_PEAKS.json.
 * ``cpu_baseline`` the CPU oracle (restated reference, OpenMP over all host cores) on a bounded
                  sample of the same workload.
 * ``--impl reference`` times the CPU oracle as the reference arm (the reference's own SYCL build
@@ -217,18 +218,19 @@ def make_props(plbm, alg, lay, w, h, steps, fui=None, wg=1024):
 
 
 def device_run(plbm, precision, alg, lay, w, h, mask, steps, warmup, tau=None, window=None):
-    """K device-resident steps; returns (ms_per_step, handler).  `window` (a list) receives the
-    wall-clock bounds of the timed steps (run_steps synchronises before it returns)."""
+    """K device-resident steps; returns (ms_per_step, launches of these steps, handler).  `window` (a
+    list) receives the wall-clock bounds of the timed steps (run_steps synchronises before it returns)."""
     props = make_props(plbm, alg, lay, w, h, steps + warmup + 10)
     if tau is not None:
         props.relaxation_time = float(tau)
     hd = plbm.create_handler(props, precision=precision, mask=mask)
     hd.run_steps(warmup)
+    launches = hd.run_launches(steps)
     t0 = time.time()
     ms = hd.run_steps(steps)
     if window is not None:
         window[:] = [t0, time.time()]
-    return ms, hd
+    return ms, launches, hd
 
 
 def e2e_run(plbm, precision, alg, lay, w, h, mask, steps):
@@ -320,10 +322,11 @@ def parity_drift(plbm, w=2000, h=500, checkpoints=(1000, 2000, 5000, 10000), tau
     return out
 
 
-# DRAM read + write bytes of one step launch, from ncu captures of the 4096^2 circle channel
-# (profiles/), per inner node; geometry scales with the domain, so traffic is proportional.
-TRAFFIC_PER_NODE = {"nptl_stream_f64_q60": 2.293e9 / (4096 * 4096), "nptl_stream_f64_fast": 2.283e9 / (4096 * 4096),
-                    "nptl_stream_f32": 1.1375e9 / (4096 * 4096), "nptl_stream_f16s": 0.5923e9 / (4096 * 4096)}
+# DRAM read + write bytes of one launch, from ncu captures of circle channels (profiles/), per inner
+# node; geometry scales with the domain, so traffic is proportional.  f64_q60 and f32: the two-step
+# kernel, whose launches move what a single step's do (2.293 / 1.1375 GB at 4096^2).
+TRAFFIC_PER_NODE = {"nptl_stream_f64_q60": 1.459e9 / (4096 * 2560), "nptl_stream_f64_fast": 2.283e9 / (4096 * 4096),
+                    "nptl_stream_f32": 1.1247e9 / (4096 * 4096)}
 
 
 def precision_study(plbm, w=1024, h=256, seed=12345, porosity=0.7, target=1e-6, max_steps=100000,
@@ -468,15 +471,13 @@ def batch_study(plbm, steps=100, precisions=("f32", "f16s"), n=256, tile=None):
         ms_pers = b.run(steps, mode="persistent")
         b.run(4, mode="per_domain")
         ms_per = b.run(steps, mode="per_domain")
-        bpn = BYTES_PER_NODE[prec]
         out[prec] = {"nodes": nodes, "tiles": tiles,
                      "tile": {"threads": [used[0], used[1] & 255], "rows_per_thread": max(1, (used[1] >> 8) & 255),
                               "vectorised_rows": bool(used[1] & plbm.BATCH_TILE_VEC),
                               "blocks_per_sm": used[2], "autotuned": tile is None or BYTES_PER_NODE[prec] != 36},
                      "mlups_persistent_graph": round(nodes / ms_graph / 1e3, 1),
                      "mlups_persistent": round(nodes / ms_pers / 1e3, 1),
-                     "mlups_per_domain_launches": round(nodes / ms_per / 1e3, 1),
-                     "hbm_gbs_persistent_graph": round(bpn * nodes / ms_graph / 1e6, 1)}
+                     "mlups_per_domain_launches": round(nodes / ms_per / 1e3, 1)}
         b.close()
     return out
 
@@ -485,7 +486,7 @@ def sweep(plbm, steps=50, warmup=5, sizes=((2000, 500), (8192, 8192)), taus=(0.5
           precisions=("f64_q60", "f64_strict")):
     """The FP64 drop-in sweep: every algorithm x data layout on the circle channel (disk of radius
     H/8 at W/4, walls, rho 1.2 / 1.0) at each size and relaxation time, device-resident steps timed
-    with CUDA events; MLUPS, algorithmic GB/s (144 B/node) and the fraction of measured HBM."""
+    with CUDA events; MLUPS, algorithmic GB/s (144 B per node and launch) and the fraction of measured HBM."""
     pk = peaks()
     rows = []
     for w, h in sizes:
@@ -494,9 +495,9 @@ def sweep(plbm, steps=50, warmup=5, sizes=((2000, 500), (8192, 8192)), taus=(0.5
             for tau in taus:
                 for alg in ("nptl", "lptl", "npol", "nsol"):
                     for lay in ("stream", "collision", "bundle"):
-                        ms, hd = device_run(plbm, prec, alg, lay, w, h, mask, steps, warmup, tau)
+                        ms, launches, hd = device_run(plbm, prec, alg, lay, w, h, mask, steps, warmup, tau)
                         hd.close()
-                        gbs = BYTES_PER_NODE[prec] * w * h / (ms * 1e-3) / 1e9
+                        gbs = BYTES_PER_NODE[prec] * w * h * launches / steps / (ms * 1e-3) / 1e9
                         rows.append({"size": f"{w}x{h}", "precision": prec, "tau": tau, "algorithm": alg,
                                      "data_layout": lay, "mlups": round(w * h / ms / 1e3, 1), "hbm_gbs": round(gbs, 1),
                                      "frac_of_hbm": round(gbs / pk["hbm_gbs"], 4)})
@@ -753,12 +754,12 @@ def main():
     # busy stretch
     clocks = ClockSampler(local).__enter__()
     run_t0 = time.time()
-    ms, hd = device_run(plbm, args.precision, args.algorithm, args.layout, w, h, mask, args.steps, args.warmup,
-                        window=window)
+    ms, launches, hd = device_run(plbm, args.precision, args.algorithm, args.layout, w, h, mask, args.steps,
+                                  args.warmup, window=window)
     barrier(world)
     ms = max_over_ranks(ms, world)
-    launches = hd.launches_per_step() * args.steps
-    bpn = BYTES_PER_NODE[args.precision]
+    # bytes a step needs: each launch reads and writes every population once
+    bpn = BYTES_PER_NODE[args.precision] * launches / args.steps
     mlups_rank = w * h / (ms * 1e-3) / 1e6
     value = mlups_rank * world
     achieved_gbs = bpn * w * h / (ms * 1e-3) / 1e9
@@ -784,12 +785,12 @@ def main():
     variants = {}
     if not args.no_variants and rank == 0:
         for prec in ("f64_q60", "f64_strict", "f64_fast", "f32", "f16s", "f16c", "bf16s"):
-            vms, vh = device_run(plbm, prec, args.algorithm, args.layout, w, h, mask, VARIANT_STEPS, 10)
+            vms, vn, vh = device_run(plbm, prec, args.algorithm, args.layout, w, h, mask, VARIANT_STEPS, 10)
             vh.close()
+            vgbs = BYTES_PER_NODE[prec] * w * h * vn / VARIANT_STEPS / vms / 1e6
             variants[prec] = {"mlups": round(w * h / vms / 1e3, 1), "ms_per_step": round(vms, 4),
                               "steps": VARIANT_STEPS,
-                              "hbm_gbs": round(BYTES_PER_NODE[prec] * w * h / vms / 1e6, 1),
-                              "frac_of_hbm": round(BYTES_PER_NODE[prec] * w * h / vms / 1e6 / pk["hbm_gbs"], 4)}
+                              "launches": vn, "hbm_gbs": round(vgbs, 1), "frac_of_hbm": round(vgbs / pk["hbm_gbs"], 4)}
         variants["ratios"] = {f"{p}_over_{q}": round(variants[p]["mlups"] / variants[q]["mlups"], 3)
                               for p in ("f16s", "f16c") for q in ("f64_q60", "f64_strict")}
 
@@ -829,13 +830,14 @@ def main():
             "config": line_config(args, world),
             "roofline": {"bound": "hbm", "achieved": round(achieved_gbs, 1), "peak": pk["hbm_gbs"], "unit": "GB/s",
                          "frac": round(achieved_gbs / pk["hbm_gbs"], 4), "traffic": traffic,
-                         # DRAM bytes the launch actually moves (ncu traffic; solid nodes move none)
-                         # over the same live launch time
-                         "dram_frac": (round(traffic / (ms * 1e-3) / 1e9 / pk["hbm_gbs"], 4)
+                         # DRAM bytes the launches actually move (ncu traffic; solid nodes move none)
+                         # over the same live time
+                         "dram_frac": (round(traffic * launches / args.steps / (ms * 1e-3) / 1e9 / pk["hbm_gbs"], 4)
                                        if traffic else None),
                          "peak_source": pk["source"],
-                         "note": ("f64_strict/f64_fast are bound by the FP64 pipe (0.5 T DP instr/s measured); "
-                                  "f64_q60 runs the update on the integer pipe")},
+                         "note": ("two-step launches of f64_q60 are bound by its integer multiplications (fmaheavy "
+                                  "pipe 74 % busy) rather than by HBM; f64_strict runs most of the update on the "
+                                  "integer pipe, f64_fast is bound by the FP64 pipe")},
             "e2e": {"value": round(e2e_mlups, 1), "unit": "MLUPS", "h2d_bytes_per_step": round(w * h / e2e_steps),
                     "d2h_bytes_per_step": round(4 * 8 * w * h / e2e_steps)},
             "gpu_launches": launches,

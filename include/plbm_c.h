@@ -189,9 +189,11 @@ int plbm_write_npy(const char *path, const double *data, unsigned rows, unsigned
 int plbm_benchmark_run(const char *settings_path, const char *benchmark_path, const char *output_root,
                        const plbm_options *opts, unsigned phases, double hbm_gbs);
 int plbm_benchmark_work_group_sizes(unsigned max_work_group_size, unsigned *out, unsigned capacity, unsigned *count);
-/* Kernel launches issued per step (for launch accounting); plain steps of the shifted forms on large
- * nptl / lptl domains run two a launch. */
+/* Kernel launches of one step that writes results (for launch accounting). */
 int plbm_launches_per_step(plbm_handler *h, unsigned *n);
+/* Kernel launches the next plbm_run_steps(h, n) issues: plain steps (no results) of the shifted forms
+ * and of the Q60 form run two a launch on large nptl / lptl domains. */
+int plbm_run_launches(plbm_handler *h, unsigned n, unsigned *launches);
 /* Algorithmic HBM bytes per node update of the hot kernel (9 loads + 9 stores). */
 int plbm_bytes_per_node(plbm_handler *h, double *bytes);
 /* Reads back the total fluid mass and momentum (FP64 reductions on the GPU). */

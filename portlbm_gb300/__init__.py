@@ -117,6 +117,7 @@ _SIGS = {
     "plbm_run_steps": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint, ctypes.POINTER(ctypes.c_double)]),
     "plbm_sync_results": (ctypes.c_int, [ctypes.c_void_p]),
     "plbm_gather_form": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)]),
+    "plbm_run_launches": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint, ctypes.POINTER(ctypes.c_uint)]),
     "plbm_launches_per_step": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint)]),
     "plbm_bytes_per_node": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_double)]),
     "plbm_mass_momentum": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_double)]),
@@ -458,6 +459,12 @@ class AlgorithmHandler:
     def launches_per_step(self) -> int:
         v = ctypes.c_uint()
         self._call("plbm_launches_per_step", ctypes.byref(v))
+        return v.value
+
+    def run_launches(self, steps: int) -> int:
+        """Kernel launches the next run_steps(steps) issues (plain steps may run two a launch)."""
+        v = ctypes.c_uint()
+        self._call("plbm_run_launches", ctypes.c_uint(steps), ctypes.byref(v))
         return v.value
 
 

@@ -1585,6 +1585,21 @@ int plbm_launches_per_step(plbm_handler *h, unsigned *n)
     return PLBM_OK;
 }
 
+int plbm_run_launches(plbm_handler *h, unsigned n, unsigned *launches)
+{
+    return guarded(h, [&] {
+        if (n == 0) {
+            *launches = 0;
+            return;
+        }
+        // as run_plain and enqueue_plain issue n - 1 plain steps, then the step with results
+        unsigned plain = n - 1, count = 1;
+        if (h->opt.use_graph && plain >= 8 && (h->iteration.load() & 1u)) --plain, ++count;
+        count += h->pair_rows ? plain / 4 * 2 + plain % 4 : plain;
+        *launches = count * (h->debug ? 3 : 1);
+    });
+}
+
 int plbm_bytes_per_node(plbm_handler *h, double *bytes)
 {
     *bytes = 18.0 * (double)storage_bytes(h->prec);

@@ -73,3 +73,18 @@ def test_frames_and_precision_change(plbm):
         assert np.array_equal(x, y)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision,w,h,pairs", [("f16s", 2401, 1511, True), ("f64_q60", 3031, 2507, True),
+                                                 ("f64_q60", 400, 100, False), ("f64_strict", 400, 100, False)])
+def test_launch_accounting(plbm, precision, w, h, pairs):
+    """run_launches follows the schedule: an odd first step, four plain steps in two launches, the rest
+    and the result step one by one."""
+    hd = handler(plbm, "nptl", "stream", precision, w, h, False)
+    for n, want in ((1, 1), (4, 4), (5, 3), (8, 6), (9, 5), (70, 36)):
+        assert hd.run_launches(n) == (want if pairs else n), n
+    hd.run_steps(1)
+    for n, want in ((8, 6), (9, 7), (10, 6)):
+        assert hd.run_launches(n) == (want if pairs else n), n
+    assert hd.run_launches(0) == 0
+    hd.close()
