@@ -324,6 +324,12 @@ int plbm_nn_relu_bwd(const void *y, void *g, long long n, void *stream);
 /* The ReLU backward of g ([P, C] bfloat16, in place: g = g where y > 0, else 0) together with the
  * bias gradient gb[c] += sum over the P pixels of the masked g[p][c] (FP32), in one pass over g. */
 int plbm_nn_relu_bwd_bias(const void *y, void *g, float *gb, long long P, int C, void *stream);
+/* The same into `out` ([N,H,W,C], P = N H W pixels), from a gradient that is formed on the way, with the
+ * values of the separate calls: GRAD g itself (out may be g); GRAD_UP2 plbm_nn_up2_bwd of g
+ * ([N,2H,2W,C]); GRAD_POOL2 plbm_nn_pool2_bwd of g ([N,H/2,W/2,C]) plus skip ([N,H,W,C]). */
+enum { PLBM_NN_GRAD = 0, PLBM_NN_GRAD_UP2 = 1, PLBM_NN_GRAD_POOL2 = 2 };
+int plbm_nn_relu_bwd_bias_from(int from, const void *g, const void *skip, const void *y, void *out, float *gb, int N, int H,
+                               int W, int C, void *stream);
 int plbm_nn_pool2(const void *x, void *y, int N, int H, int W, int C, void *stream);
 int plbm_nn_pool2_bwd(const void *gy, void *gx, int N, int H, int W, int C, void *stream);
 int plbm_nn_up2(const void *x, void *y, int N, int H, int W, int C, void *stream);

@@ -398,56 +398,25 @@ __device__ __forceinline__ uint4 relu_mask8(uint4 yv, uint4 gv)
     return gv;
 }
 
-// gb[c] += sum over the P pixels of g[p][c]: thread (pixel lane q, unit u) of a block of
-// R = blockDim.x / CU pixel lanes sums unit u of every (R * gridDim.x)-th pixel; the block's lanes
-// are then added per channel in shared memory, one atomic per channel and block.  RELU: the ReLU
-// backward first, in place (g = g * (y > 0)), and the masked values summed: one pass over g.
-template <bool RELU>
-__global__ void k_bias_grad_v(const uint4 *y, uint4 *g, float *gb, unsigned P, int CU)
-{
-    extern __shared__ float red[];
-    const int R = blockDim.x / CU, q = threadIdx.x / CU, u = threadIdx.x - q * CU;
-    float s[8] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
-    if (q < R)
-        for (unsigned p = blockIdx.x * (unsigned)R + q; p < P; p += gridDim.x * (unsigned)R) {
-            const size_t i = (size_t)p * CU + u;
-            uint4 gv = g[i];
-            if constexpr (RELU) {
-                gv = relu_mask8(y[i], gv);
-                g[i] = gv;
-            }
-            float f[8];
-            unpack8(gv, f);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) s[e] += f[e];
-        }
-    if (q < R)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) red[threadIdx.x * 8 + e] = s[e];
-    __syncthreads();
-    for (int k = threadIdx.x; k < CU * 8; k += blockDim.x) {
-        float t = 0.f;
-        for (int qq = 0; qq < R; ++qq) t += red[qq * CU * 8 + k];
-        atomicAdd(&gb[k], t);
-    }
-}
-
 __global__ void k_relu_bwd_v(const uint4 *y, uint4 *g, unsigned n8)
 {
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += gridDim.x * blockDim.x) g[i] = relu_mask8(y[i], g[i]);
 }
 
+__device__ __forceinline__ uint4 add8(uint4 a, uint4 b)
+{
+    float fa[8], fb[8];
+    unpack8(a, fa);
+    unpack8(b, fb);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) fa[e] += fb[e];
+    return pack8(fa);
+}
+
 __global__ void k_add_v(const uint4 *a, const uint4 *b, uint4 *y, unsigned n8)
 {
     nn_begin();
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += gridDim.x * blockDim.x) {
-        float fa[8], fb[8];
-        unpack8(a[i], fa);
-        unpack8(b[i], fb);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) fa[e] += fb[e];
-        y[i] = pack8(fa);
-    }
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += gridDim.x * blockDim.x) y[i] = add8(a[i], b[i]);
 }
 
 // Output unit i of [N][H][W][CU] (H, W the output size) from input unit (n, yy / 2, xx / 2).
@@ -461,26 +430,28 @@ __global__ void k_up2_v(const uint4 *x, uint4 *y, unsigned N, unsigned H, unsign
     }
 }
 
-// Input-gradient unit i of [N][H][W][CU] (H, W the input size): the sum of its four output units.
+// Unit cu of input-gradient pixel p of [N][H][W][CU] (H, W the input size): the sum of its four output units.
+__device__ __forceinline__ uint4 up2_bwd_unit(const uint4 *gy, unsigned p, unsigned cu, unsigned H, unsigned W, unsigned CU)
+{
+    const unsigned x = p % W, t2 = p / W, yv = t2 % H, n = t2 / H;
+    const size_t b = ((size_t)(n * 2 * H + 2 * yv) * (2 * W) + 2 * x) * CU + cu, row = (size_t)2 * W * CU;
+    const uint4 u[4] = { gy[b], gy[b + CU], gy[b + row], gy[b + row + CU] };
+    float s[8], f[8];
+    unpack8(u[0], s);
+#pragma unroll
+    for (int k = 1; k < 4; ++k) {
+        unpack8(u[k], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] += f[e];
+    }
+    return pack8(s);
+}
+
 __global__ void k_up2_bwd_v(const uint4 *gy, uint4 *gx, unsigned N, unsigned H, unsigned W, unsigned CU)
 {
     const unsigned total = N * H * W * CU;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const unsigned cu = i % CU, t = i / CU, x = t % W, t2 = t / W, yv = t2 % H, n = t2 / H;
-        const size_t b = ((size_t)(n * 2 * H + 2 * yv) * (2 * W) + 2 * x) * CU + cu, row = (size_t)2 * W * CU;
-        float s[8], f[8];
-        unpack8(gy[b], s);
-        unpack8(gy[b + CU], f);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) s[e] += f[e];
-        unpack8(gy[b + row], f);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) s[e] += f[e];
-        unpack8(gy[b + row + CU], f);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) s[e] += f[e];
-        gx[i] = pack8(s);
-    }
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+        gx[i] = up2_bwd_unit(gy, i / CU, i % CU, H, W, CU);
 }
 
 // Output unit i of [N][H/2][W/2][CU] (H, W the input size): the mean of its four input units.
@@ -506,17 +477,65 @@ __global__ void k_pool2_v(const uint4 *x, uint4 *y, unsigned N, unsigned H, unsi
     }
 }
 
-// Input-gradient unit i of [N][H][W][CU] (H, W the input size): a quarter of its pooled unit.
+// Unit cu of input-gradient pixel p of [N][H][W][CU] (H, W the input size): a quarter of its pooled unit.
+__device__ __forceinline__ uint4 pool2_bwd_unit(const uint4 *gy, unsigned p, unsigned cu, unsigned H, unsigned W, unsigned CU)
+{
+    const unsigned x = p % W, t2 = p / W, yv = t2 % H, n = t2 / H;
+    float f[8];
+    unpack8(gy[((size_t)(n * (H / 2) + yv / 2) * (W / 2) + x / 2) * CU + cu], f);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] *= 0.25f;
+    return pack8(f);
+}
+
 __global__ void k_pool2_bwd_v(const uint4 *gy, uint4 *gx, unsigned N, unsigned H, unsigned W, unsigned CU)
 {
     const unsigned total = N * H * W * CU;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const unsigned cu = i % CU, t = i / CU, x = t % W, t2 = t / W, yv = t2 % H, n = t2 / H;
-        float f[8];
-        unpack8(gy[((size_t)(n * (H / 2) + yv / 2) * (W / 2) + x / 2) * CU + cu], f);
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+        gx[i] = pool2_bwd_unit(gy, i / CU, i % CU, H, W, CU);
+}
+
+// gb[c] += sum over the P pixels of a gradient: thread (pixel lane q, unit u) of a block of
+// R = blockDim.x / CU pixel lanes sums unit u of every (R * gridDim.x)-th pixel; the block's lanes
+// are then added per channel in shared memory, one atomic per channel and block.  RELU: the ReLU
+// backward first (g = g * (y > 0)), and the masked values stored to `out` and summed.  FROM says
+// where the gradient comes from: the buffer src (out may be the same), the up-sampling's backward of
+// src, or the pooling's backward of src plus the skip gradient.
+// Bound by memory: these passes were kernels of their own (and a copy of the skip gradient), which
+// wrote and read the gradient again at every level; with them here each level's gradient is written once.
+// 16 x 256^2 training step: 2530 -> 2430 us.
+template <int FROM, bool RELU>
+__global__ void k_bias_grad_v(const uint4 *src, const uint4 *skip, const uint4 *y, uint4 *out, float *gb, unsigned P,
+                              unsigned H, unsigned W, int CU)
+{
+    extern __shared__ float red[];
+    nn_begin();
+    const int R = blockDim.x / CU, q = threadIdx.x / CU, u = threadIdx.x - q * CU;
+    float s[8] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
+    if (q < R)
+        for (unsigned p = blockIdx.x * (unsigned)R + q; p < P; p += gridDim.x * (unsigned)R) {
+            const size_t i = (size_t)p * CU + u;
+            uint4 gv;
+            if constexpr (FROM == PLBM_NN_GRAD_UP2) gv = up2_bwd_unit(src, p, u, H, W, CU);
+            else if constexpr (FROM == PLBM_NN_GRAD_POOL2) gv = add8(pool2_bwd_unit(src, p, u, H, W, CU), skip[i]);
+            else gv = src[i];
+            if constexpr (RELU) {
+                gv = relu_mask8(y[i], gv);
+                out[i] = gv;
+            }
+            float f[8];
+            unpack8(gv, f);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] *= 0.25f;
-        gx[i] = pack8(f);
+            for (int e = 0; e < 8; ++e) s[e] += f[e];
+        }
+    if (q < R)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) red[threadIdx.x * 8 + e] = s[e];
+    __syncthreads();
+    for (int k = threadIdx.x; k < CU * 8; k += blockDim.x) {
+        float t = 0.f;
+        for (int qq = 0; qq < R; ++qq) t += red[qq * CU * 8 + k];
+        atomicAdd(&gb[k], t);
     }
 }
 
@@ -530,22 +549,24 @@ bool vec8(int C, long long elems, const void *a, const void *b = nullptr, const 
     return C % 8 == 0 && elems % 8 == 0 && elems / 8 < (1ll << 31) && al(a) && al(b) && al(c);
 }
 
+template <int FROM, bool RELU>
+int bias_grad_v(const void *src, const void *skip, const void *y, void *out, float *gb, long long P, int H, int W, int C,
+                cudaStream_t s)
+{
+    const int CU = C / 8, threads = (256 / CU) * CU;
+    const long long R = threads / CU;
+    const unsigned blocks = (unsigned)((P + R - 1) / R < 152 * 4 ? (P + R - 1) / R : 152 * 4);
+    return launched(nn_launch(k_bias_grad_v<FROM, RELU>, blocks, threads, threads * 8 * sizeof(float), s, (const uint4 *)src,
+                              (const uint4 *)skip, (const uint4 *)y, (uint4 *)out, gb, (unsigned)P, H, W, CU));
+}
+
 // gb[c] += sum over the P pixels of g[p][c]; with y, the ReLU backward of g first, in place (the
 // 16-byte kernel needs C a multiple of 8 and aligned buffers; y without them is applied by the caller).
 int bias_grad(const void *y, void *g, float *gb, long long P, int C, cudaStream_t s)
 {
-    if (vec8(C, P * C, g, y)) {
-        const int CU = C / 8, threads = (256 / CU) * CU;
-        const long long R = threads / CU;
-        const int blocks = (int)((P + R - 1) / R < 152 * 4 ? (P + R - 1) / R : 152 * 4);
-        if (y)
-            k_bias_grad_v<true><<<blocks, threads, threads * 8 * sizeof(float), s>>>((const uint4 *)y, (uint4 *)g, gb,
-                                                                                   (unsigned)P, CU);
-        else
-            k_bias_grad_v<false><<<blocks, threads, threads * 8 * sizeof(float), s>>>(nullptr, (uint4 *)g, gb,
-                                                                                    (unsigned)P, CU);
-        return cudaGetLastError() == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
-    }
+    if (vec8(C, P * C, g, y))
+        return y ? bias_grad_v<PLBM_NN_GRAD, true>(g, nullptr, y, g, gb, P, 1, 1, C, s)
+                 : bias_grad_v<PLBM_NN_GRAD, false>(g, nullptr, nullptr, nullptr, gb, P, 1, 1, C, s);
     const long long gx = (P + 7) / 8 < 1024 ? (P + 7) / 8 : 1024;
     dim3 grid((unsigned)gx, (unsigned)((C + 31) / 32));
     k_bias_grad<<<grid, 256, 0, s>>>((const __nv_bfloat16 *)g, gb, P, C);
@@ -664,6 +685,32 @@ int plbm_nn_relu_bwd_bias(const void *y, void *g, float *gb, long long P, int C,
         return rc == PLBM_OK ? bias_grad(nullptr, g, gb, P, C, (cudaStream_t)stream) : rc;
     }
     return bias_grad(y, g, gb, P, C, (cudaStream_t)stream);
+}
+
+int plbm_nn_relu_bwd_bias_from(int from, const void *g, const void *skip, const void *y, void *out, float *gb, int N, int H,
+                               int W, int C, void *stream)
+{
+    const long long P = (long long)N * H * W;
+    const bool pool = from == PLBM_NN_GRAD_POOL2, up = from == PLBM_NN_GRAD_UP2;
+    if (P <= 0 || C <= 0 || !g || !y || !out || !gb || (pool && !skip)) return PLBM_ERR_ARGUMENT;
+    if (!pool && !up && from != PLBM_NN_GRAD) return PLBM_ERR_ARGUMENT;
+    cudaStream_t s = (cudaStream_t)stream;
+    // the 16-byte kernels; a block has at least one pixel lane, and every pixel a pooled one
+    if (C <= 2048 && vec8(C, P * C * (up ? 4 : 1), g, y, out) && vec8(C, P * C, skip) && !(pool && (H % 2 || W % 2))) {
+        if (pool) return bias_grad_v<PLBM_NN_GRAD_POOL2, true>(g, skip, y, out, gb, P, H, W, C, s);
+        if (up) return bias_grad_v<PLBM_NN_GRAD_UP2, true>(g, nullptr, y, out, gb, P, H, W, C, s);
+        return bias_grad_v<PLBM_NN_GRAD, true>(g, nullptr, y, out, gb, P, 1, 1, C, s);
+    }
+    int rc;
+    if (pool) {
+        rc = plbm_nn_pool2_bwd(g, out, N, H, W, C, stream);
+        if (rc == PLBM_OK) rc = plbm_nn_add(out, skip, out, P * C, stream);
+    } else if (up) {
+        rc = plbm_nn_up2_bwd(g, out, N, H, W, C, stream);
+    } else {
+        rc = g == out ? PLBM_OK : launched(cudaMemcpyAsync(out, g, (size_t)P * C * 2, cudaMemcpyDeviceToDevice, s));
+    }
+    return rc == PLBM_OK ? plbm_nn_relu_bwd_bias(y, out, gb, P, C, stream) : rc;
 }
 
 int plbm_nn_relu_bwd(const void *y, void *g, long long n, void *stream)

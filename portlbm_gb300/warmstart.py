@@ -43,6 +43,7 @@ ENC = [(C_IN, 32), (32, 32), (32, 64), (64, 64), (64, 96), (96, 96), (96, 128), 
 DEC = [(128, 128), (128, 128), (128, 96), (96, 96), (96, 64), (64, 64), (64, 32), (32, 32)]
 HEAD = (32, 3)
 WIDTHS = [32, 64, 96, 128, 128]
+GRAD, GRAD_UP2, GRAD_POOL2 = 0, 1, 2     # gradient sources of plbm_nn_relu_bwd_bias_from
 
 
 def _fns():
@@ -56,6 +57,7 @@ def _fns():
         "plbm_nn_conv_wgrad": [vp, vp, vp, vp, i, i, i, i, i, vp],
         "plbm_nn_relu_bwd": [vp, vp, ll, vp],
         "plbm_nn_relu_bwd_bias": [vp, vp, vp, ll, i, vp],
+        "plbm_nn_relu_bwd_bias_from": [i, vp, vp, vp, vp, vp, i, i, i, i, vp],
         "plbm_nn_pool2": [vp, vp, i, i, i, i, vp],
         "plbm_nn_pool2_bwd": [vp, vp, i, i, i, i, vp],
         "plbm_nn_up2": [vp, vp, i, i, i, i, vp],
@@ -272,17 +274,24 @@ class NeuralOperator:
         self.acts, self.shape = Activations(x, work, plan, out), (n, h, w)
         return out
 
-    def _conv_bwd(self, layer, x, y, gy, n, h, w, need_gx=True):
-        gb = layer.gb.data_ptr()
-        if layer.relu:   # the ReLU backward and the bias gradient in one pass over the gradient
-            _ok(self.lib.plbm_nn_relu_bwd_bias(y.data_ptr(), gy.data_ptr(), gb, n * h * w, layer.cout, self._s))
-            gb = None
-        _ok(self.lib.plbm_nn_conv_wgrad(x.data_ptr(), gy.data_ptr(), layer.gw.data_ptr(), gb, n, h, w, layer.cin,
-                                        layer.cout, self._s))
+    def _relu_bwd(self, layer, y, n, h, w, g, source=GRAD, skip=None, out=None):
+        """The gradient of a layer's convolution from that of its output, formed on the way from g
+        (see GRAD, GRAD_UP2, GRAD_POOL2), and the layer's bias gradient, in one pass."""
+        out = self._buf(n, h, w, layer.cout) if out is None else out
+        _ok(self.lib.plbm_nn_relu_bwd_bias_from(source, g.data_ptr(), skip.data_ptr() if skip is not None else None,
+                                                y.data_ptr(), out.data_ptr(), layer.gb.data_ptr(), n, h, w, layer.cout,
+                                                self._s))
+        return out
+
+    def _conv_bwd(self, layer, x, g, n, h, w, need_gx=True):
+        """The weight gradient (of a layer without ReLU also the bias gradient) and the input gradient."""
+        _ok(self.lib.plbm_nn_conv_wgrad(x.data_ptr(), g.data_ptr(), layer.gw.data_ptr(),
+                                        None if layer.relu else layer.gb.data_ptr(), n, h, w, layer.cin, layer.cout,
+                                        self._s))
         if not need_gx:
             return None
         gx = self._buf(n, h, w, layer.cin)
-        _ok(self.lib.plbm_nn_conv_dgrad_pre(gy.data_ptr(), layer.wb.data_ptr(), layer.wbt.data_ptr(), gx.data_ptr(),
+        _ok(self.lib.plbm_nn_conv_dgrad_pre(g.data_ptr(), layer.wb.data_ptr(), layer.wbt.data_ptr(), gx.data_ptr(),
                                             n, h, w, layer.cin, layer.cout, self._s))
         return gx
 
@@ -292,30 +301,23 @@ class NeuralOperator:
         _ok(self.lib.plbm_nn_flip_layers(p.wb.data_ptr(), p.wbt.data_ptr(), self._segs.data_ptr(), len(self.layers),
                                          self._max_elems, self._s))
         a, (n, h, w) = self.acts, self.shape
-        g = self._conv_bwd(self.head, a["d0b"], a["out"], gout, n, h, w)
+        g, source = self._conv_bwd(self.head, a["d0b"], gout, n, h, w), GRAD
         gskip = {}
-        sizes = {lvl: (h >> lvl, w >> lvl) for lvl in range(5)}
-        for k, lvl in enumerate((0, 1, 2, 3)):
-            kk = 3 - k
-            sh, sw = sizes[lvl]
-            gs = self._conv_bwd(self.dec[2 * kk + 1], a[f"s{lvl}"], a[f"d{lvl}b"], g, n, sh, sw)
-            gskip[lvl] = gs                                     # the skip addition passes g to both inputs
-            gu = self._conv_bwd(self.dec[2 * kk], a[f"u{lvl}"], a[f"d{lvl}a"], gs.clone(), n, sh, sw)
-            ch, cw = sizes[lvl + 1]
-            g = self._buf(n, ch, cw, gu.shape[-1])
-            _ok(self.lib.plbm_nn_up2_bwd(gu.data_ptr(), g.data_ptr(), n, ch, cw, gu.shape[-1], self._s))
-        for lvl in (4, 3, 2, 1, 0):
-            hh, ww = sizes[lvl]
-            if lvl < 4:
-                # gradient of e{lvl}b: skip gradient + pooled path gradient
-                gp = self._buf(n, hh, ww, g.shape[-1])
-                _ok(self.lib.plbm_nn_pool2_bwd(g.data_ptr(), gp.data_ptr(), n, hh, ww, g.shape[-1], self._s))
-                gb_ = self._buf(n, hh, ww, g.shape[-1])
-                _ok(self.lib.plbm_nn_add(gp.data_ptr(), gskip[lvl].data_ptr(), gb_.data_ptr(), gb_.numel(), self._s))
-                g = gb_
-            xin = a["in"] if lvl == 0 else a[f"p{lvl - 1}"]
-            ga = self._conv_bwd(self.enc[2 * lvl + 1], a[f"e{lvl}a"], a[f"e{lvl}b"], g, n, hh, ww)
-            g = self._conv_bwd(self.enc[2 * lvl], xin, a[f"e{lvl}a"], ga, n, hh, ww, need_gx=lvl > 0)
+        for lvl in range(LEVELS - 1):
+            first, second = self.dec[2 * (LEVELS - 2 - lvl)], self.dec[2 * (LEVELS - 2 - lvl) + 1]
+            size = n, h >> lvl, w >> lvl
+            g = self._relu_bwd(second, a[f"d{lvl}b"], *size, g, source, out=g if source == GRAD else None)
+            gskip[lvl] = self._conv_bwd(second, a[f"s{lvl}"], g, *size)   # passes to both inputs of the skip addition
+            g = self._relu_bwd(first, a[f"d{lvl}a"], *size, gskip[lvl])
+            g, source = self._conv_bwd(first, a[f"u{lvl}"], g, *size), GRAD_UP2
+        for lvl in reversed(range(LEVELS)):
+            first, second = self.enc[2 * lvl], self.enc[2 * lvl + 1]
+            size = n, h >> lvl, w >> lvl
+            g = self._relu_bwd(second, a[f"e{lvl}b"], *size, g, source, gskip.get(lvl))
+            ga = self._conv_bwd(second, a[f"e{lvl}a"], g, *size)
+            ga = self._relu_bwd(first, a[f"e{lvl}a"], *size, ga, out=ga)
+            g = self._conv_bwd(first, a["in"] if lvl == 0 else a[f"p{lvl - 1}"], ga, *size, need_gx=lvl > 0)
+            source = GRAD_POOL2
 
     def zero_grad(self):
         self.params.g.zero_()
