@@ -56,3 +56,38 @@ def test_arguments_are_checked(plbm):
     p = t.data_ptr()
     for source, skip, n in ((3, p, 1), (ws.GRAD_POOL2, None, 1), (ws.GRAD, None, 0)):
         assert lib.plbm_nn_relu_bwd_bias_from(source, p, skip, p, p, gb.data_ptr(), n, 2, 2, 8, None) != 0
+
+
+@pytest.mark.parametrize("p,c", [(8, 1), (8, 3), (1000, 3), (65536 * 3 + 8, 3), (4096, 5), (24, 60), (120000, 12), (77, 3)])
+def test_narrow_bias_gradient(plbm, p, c):
+    """The bias gradient that comes with the weight gradient of a layer without ReLU, a few channels wide."""
+    from portlbm_gb300 import warmstart as ws
+    lib = ws._fns()
+    gen = torch.Generator(device="cuda").manual_seed(p + c)
+    g = torch.randn((1, 1, p, c), generator=gen, device="cuda").to(torch.bfloat16)
+    x = torch.zeros((1, 1, p, 1), dtype=torch.bfloat16, device="cuda")
+    gw, start = torch.zeros(c * 9, device="cuda"), torch.randn(c, generator=gen, device="cuda")
+    gb = start.clone()
+    assert lib.plbm_nn_conv_wgrad(x.data_ptr(), g.data_ptr(), gw.data_ptr(), gb.data_ptr(), 1, 1, p, 1, c, None) == 0
+    terms = g.double().reshape(-1, c)
+    bound = (terms.abs().sum(0) + start.double().abs()) * (p + 1) * 2.0 ** -24
+    assert ((gb.double() - start.double() - terms.sum(0)).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("p,c", [(8, 1), (8, 3), (104, 3), (77, 3), (65536, 3), (1000, 5), (333, 16), (640000, 3)])
+def test_mean_squared_error(plbm, p, c):
+    from portlbm_gb300 import warmstart as ws
+    lib = ws._fns()
+    gen = torch.Generator(device="cuda").manual_seed(p + c)
+    pred = torch.randn((p, c), generator=gen, device="cuda").to(torch.bfloat16)
+    target = torch.randn((p, c), generator=gen, device="cuda")
+    mask = (torch.rand(p, generator=gen, device="cuda") < 0.3).to(torch.int8)
+    inv = 1.0 / max(1, int((mask == 0).sum()) * c)
+    grad, loss = torch.empty_like(pred), torch.zeros(1, device="cuda")
+    assert lib.plbm_nn_mse(pred.data_ptr(), target.data_ptr(), mask.data_ptr(), grad.data_ptr(), loss.data_ptr(), p, c,
+                           inv, None) == 0
+    d = torch.where((mask == 0)[:, None], pred.float() - target, 0.0)
+    inv32 = torch.tensor(inv, dtype=torch.float32, device="cuda")
+    assert torch.equal(grad, (2.0 * d * inv32).to(torch.bfloat16))
+    want = (d.double() ** 2).sum() * inv
+    assert abs(loss.double() - want) <= want * (p * c + 3) * 2.0 ** -24
