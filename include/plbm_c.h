@@ -362,14 +362,14 @@ int plbm_nn_adam_dev(float *w, const float *g, float *m, float *v, void *w_bf16,
 /* Network input [N,H,W,C] (C >= 4): channel 0 the int8 solid mask, channels 1..3 the per-sample
  * scalars features[3n..3n+2] as constant planes, further channels zero. */
 /* 1 when plbm_nn_conv_fwd runs the shape (input channels Cin, output channels Cout) on tcgen05:
- * W a multiple of 128 or a power of two below 128 with H a multiple of 128 / W, and either Cin a
- * multiple of 32 with Cout <= 128 (TMA-fed kernel) or 9 * Cin <= 64 with Cout <= 64 (kernel whose
+ * Cin a multiple of 32 with Cout <= 128 (TMA-fed kernel, any image), or 9 * Cin <= 64 with Cout <= 64
+ * and W a multiple of 128 or a power of two below 128 with H a multiple of 128 / W (kernel whose
  * threads write the im2col tile).  plbm_nn_conv_dgrad uses it with the two channel counts
- * exchanged.  Other shapes run the mma.sync kernel. */
+ * exchanged.  Other shapes, and buffers that do not start on 16 bytes, run the mma.sync kernel. */
 int plbm_nn_conv_on_tensor_cores(int H, int W, int Cin, int Cout);
-/* 1 when plbm_nn_conv_wgrad runs the shape on tcgen05: the image tiling above, Cout <= 128, and
- * either Cin a multiple of 32 up to 128 (TMA-fed input tiles) or Cin <= 32 (im2col tiles written by
- * the CTA's threads). */
+/* 1 when plbm_nn_conv_wgrad runs the shape on tcgen05: Cout <= 128, and either Cin a multiple of 32 up
+ * to 128 (TMA-fed input tiles) or Cin <= 32 on the images above (im2col tiles written by the CTA's
+ * threads). */
 int plbm_nn_wgrad_on_tensor_cores(int H, int W, int Cin, int Cout);
 /* Synchronises the device and reports whether a tensor-core convolution gave up on a wait (its
  * output is then invalid); clears the flag. */

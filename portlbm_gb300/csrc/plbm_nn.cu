@@ -17,7 +17,7 @@
 // Tensor-core convolution (plbm_nn_tc.cu).
 bool plbm_nn_tc_supported(int H, int W, int Cin, int Cout);
 int plbm_nn_tc_conv(const void *x, const void *w, const float *bias, void *y, int N, int H, int W, int Cin, int Cout,
-                    int relu, cudaStream_t s);
+                    int relu, bool dgrad, cudaStream_t s);
 int plbm_nn_tc_flip(const void *w, void *wt, int Cin, int Cout, cudaStream_t s);
 bool plbm_nn_tc_wgrad_supported(int H, int W, int Cin, int Cout);
 int plbm_nn_tc_wgrad(const void *x, const void *g, float *gw, float *gb, int N, int H, int W, int Cin, int Cout,
@@ -639,6 +639,12 @@ int bias_grad(const void *y, void *g, float *gb, long long P, int C, cudaStream_
     return cudaGetLastError() == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
 }
 
+// TMA and the kernels' 16-byte accesses need buffers that start on a 16-byte boundary; others take k_conv.
+bool aligned16(const void *a, const void *b, const void *c)
+{
+    return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15u) == 0;
+}
+
 template <int MODE>
 int run_conv(ConvArgs a, cudaStream_t s)
 {
@@ -659,9 +665,10 @@ extern "C" {
 int plbm_nn_conv_fwd(const void *x, const void *w, const float *bias, void *y, int N, int H, int W, int Cin,
                      int Cout, int relu, void *stream)
 {
-    if (plbm_nn_tc_supported(H, W, Cin, Cout))
-        return plbm_nn_tc_conv(x, w, bias, y, N, H, W, Cin, Cout, relu, (cudaStream_t)stream);
-    if (plbm_nn_tc_small_supported(H, W, Cin, Cout))
+    const bool aligned = aligned16(x, w, y);
+    if (aligned && plbm_nn_tc_supported(H, W, Cin, Cout))
+        return plbm_nn_tc_conv(x, w, bias, y, N, H, W, Cin, Cout, relu, false, (cudaStream_t)stream);
+    if (aligned && plbm_nn_tc_small_supported(H, W, Cin, Cout))
         return plbm_nn_tc_small_conv(x, w, bias, y, N, H, W, Cin, Cout, relu, (cudaStream_t)stream);
     ConvArgs a{};
     a.x = (const __nv_bfloat16 *)x; a.w = (const __nv_bfloat16 *)w; a.bias = bias; a.y = (__nv_bfloat16 *)y;
@@ -681,9 +688,10 @@ int plbm_nn_flip_layers(const void *w, void *wt, const int *segs, int layers, in
 int plbm_nn_conv_dgrad_pre(const void *g, const void *w, const void *wt, void *gx, int N, int H, int W, int Cin,
                            int Cout, void *stream)
 {
-    const bool tma = plbm_nn_tc_supported(H, W, Cout, Cin);
-    if (tma) return plbm_nn_tc_conv(g, wt, nullptr, gx, N, H, W, Cout, Cin, 0, (cudaStream_t)stream);
-    if (plbm_nn_tc_small_supported(H, W, Cout, Cin))
+    const bool aligned = aligned16(g, wt, gx);
+    if (aligned && plbm_nn_tc_supported(H, W, Cout, Cin))
+        return plbm_nn_tc_conv(g, wt, nullptr, gx, N, H, W, Cout, Cin, 0, true, (cudaStream_t)stream);
+    if (aligned && plbm_nn_tc_small_supported(H, W, Cout, Cin))
         return plbm_nn_tc_small_conv(g, wt, nullptr, gx, N, H, W, Cout, Cin, 0, (cudaStream_t)stream);
     return plbm_nn_conv_dgrad(g, w, gx, N, H, W, Cin, Cout, stream);
 }
@@ -694,7 +702,7 @@ int plbm_nn_conv_dgrad(const void *g, const void *w, void *gx, int N, int H, int
     // tensor cores (the TMA one, or for a narrow gradient the one with thread-written tiles), with
     // the re-laid-out weights in a buffer kept for the process
     const bool tma = plbm_nn_tc_supported(H, W, Cout, Cin);
-    if (tma || plbm_nn_tc_small_supported(H, W, Cout, Cin)) {
+    if (aligned16(g, gx, nullptr) && (tma || plbm_nn_tc_small_supported(H, W, Cout, Cin))) {
         // a buffer that grows is replaced, not freed: a CUDA graph captured earlier may still
         // launch with the old pointer
         static std::mutex mu;
@@ -710,7 +718,7 @@ int plbm_nn_conv_dgrad(const void *g, const void *w, void *gx, int N, int H, int
         }
         const int rc = plbm_nn_tc_flip(w, wt, Cin, Cout, (cudaStream_t)stream);
         if (rc != PLBM_OK) return rc;
-        return tma ? plbm_nn_tc_conv(g, wt, nullptr, gx, N, H, W, Cout, Cin, 0, (cudaStream_t)stream)
+        return tma ? plbm_nn_tc_conv(g, wt, nullptr, gx, N, H, W, Cout, Cin, 0, true, (cudaStream_t)stream)
                    : plbm_nn_tc_small_conv(g, wt, nullptr, gx, N, H, W, Cout, Cin, 0, (cudaStream_t)stream);
     }
     ConvArgs a{};
@@ -724,11 +732,12 @@ int plbm_nn_conv_wgrad(const void *x, const void *g, float *gw, float *gb, int N
                        void *stream)
 {
     int rc;
-    if (plbm_nn_tc_wgrad_supported(H, W, Cin, Cout)) {
+    const bool aligned = aligned16(x, g, nullptr);
+    if (aligned && plbm_nn_tc_wgrad_supported(H, W, Cin, Cout)) {
         int bias_done = 0;
         rc = plbm_nn_tc_wgrad(x, g, gw, gb, N, H, W, Cin, Cout, &bias_done, (cudaStream_t)stream);
         if (bias_done) gb = nullptr;   // the bias gradient came with the weight gradient
-    } else if (plbm_nn_tc_small_wgrad_supported(H, W, Cin, Cout)) {
+    } else if (aligned && plbm_nn_tc_small_wgrad_supported(H, W, Cin, Cout)) {
         rc = plbm_nn_tc_small_wgrad(x, g, gw, N, H, W, Cin, Cout, (cudaStream_t)stream);
     } else {
         ConvArgs a{};

@@ -14,10 +14,10 @@ __device__ __forceinline__ void nn_begin()
 }
 
 template <typename... P, typename... A>
-inline cudaError_t nn_launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args)
+inline cudaError_t nn_launch(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A... args)
 {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;

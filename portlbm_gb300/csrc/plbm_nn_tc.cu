@@ -85,6 +85,15 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(unsigned addr)
            ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
 }
 
+// The same with rows of 32 channels (64 bytes) or 64 channels (128 bytes, 128-byte swizzle, 8-row groups 1 KB).
+template <int KB>
+__device__ __forceinline__ uint64_t smem_desc_rows(unsigned addr)
+{
+    if (KB == TC_KB) return smem_desc_sw64(addr);
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
 // Instruction descriptor, kind::f16: FP32 accumulator, BF16 A and B, both K-major, N x M = npad x 128.
 __device__ __forceinline__ unsigned instr_desc(int npad)
 {
@@ -143,13 +152,15 @@ __device__ __forceinline__ void store_row16(__nv_bfloat16 *out, int c0, int C, c
 struct TcArgs {
     __nv_bfloat16 *y;
     const float *bias;      // may be null
-    int N, H, W, Cin, Cout, npad, relu;
+    int N, H, W, Cin, Cout, npad, relu;   // npad: output channels of a CTA (blockIdx.y: which ones)
     int BW, BH, tiles_x, tiles_y;
     int stage_bytes;        // A tile + the B tile rounded up to 1024 B
     int stages;
+    int last_tap_first;     // accumulate the taps from the last to the first
     int *err;
 };
 
+template <int KB>   // channels per K block: 32 or 64
 __global__ void __launch_bounds__(128, 4)
 k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, TcArgs a)
 {
@@ -175,8 +186,13 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
                      "r"(ncols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (threadIdx.x == 32) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&xmap)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&wmap)) : "memory");
+    }
     nn_begin();
-    stage_bias(s_bias, a.bias, a.Cout, a.npad);
+    const int co0 = blockIdx.y * a.npad;       // the CTA's first output channel
+    stage_bias(s_bias, a.bias ? a.bias + co0 : nullptr, a.Cout - co0, a.npad);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -187,8 +203,8 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
     const int per_img = a.tiles_x * a.tiles_y;
     const int n = tile / per_img, t2 = tile % per_img;
     const int y0 = (t2 / a.tiles_x) * a.BH, x0 = (t2 % a.tiles_x) * a.BW;
-    const int kblocks = a.Cin / TC_KB, iters = 9 * kblocks;
-    const unsigned bbytes = (unsigned)a.npad * TC_KB * 2;
+    const int kblocks = a.Cin / KB, iters = 9 * kblocks;
+    const unsigned abytes = TC_BM * KB * 2, bbytes = (unsigned)a.npad * KB * 2;
 
     if (warp == 0 && lane == 0) {              // producer: TMA loads
         for (int it = 0, s = 0, round = 0; it < iters; ++it, s = s + 1 == a.stages ? (++round, 0) : s + 1) {
@@ -196,13 +212,13 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
                 counts[2] = 1;
                 break;
             }
-            const int tap = it / kblocks, kb = it % kblocks;
+            const int kb = it % kblocks, tap = a.last_tap_first ? 8 - it / kblocks : it / kblocks;
             const int dy = tap / 3 - 1, dx = tap % 3 - 1;
             unsigned char *st = smem + s * a.stage_bytes;
             const unsigned bar = smem_u32(&full[s]);
-            mbar_expect_tx(bar, (unsigned)TC_A_BYTES + bbytes);
-            tma_load_4d(smem_u32(st), &xmap, kb * TC_KB, x0 + dx, y0 + dy, n, bar);
-            tma_load_3d(smem_u32(st + TC_A_BYTES), &wmap, kb * TC_KB, tap, 0, bar);
+            mbar_expect_tx(bar, abytes + bbytes);
+            tma_load_4d(smem_u32(st), &xmap, kb * KB, x0 + dx, y0 + dy, n, bar);
+            tma_load_3d(smem_u32(st) + abytes, &wmap, kb * KB, tap, co0, bar);
             counts[0] = it + 1;
         }
     } else if (warp == 1 && lane == 0) {       // MMA issuer
@@ -213,10 +229,10 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned abase = smem_u32(smem + s * a.stage_bytes), bbase = abase + TC_A_BYTES;
+            const unsigned abase = smem_u32(smem + s * a.stage_bytes), bbase = abase + abytes;
 #pragma unroll
-            for (int k = 0; k < TC_KB / 16; ++k)   // K = 16 per MMA: +32 B along the swizzled row
-                umma(tmem, smem_desc_sw64(abase + 32 * k), smem_desc_sw64(bbase + 32 * k), idesc, it > 0 || k > 0);
+            for (int k = 0; k < KB / 16; ++k)   // K = 16 per MMA: +32 B along the swizzled row
+                umma(tmem, smem_desc_rows<KB>(abase + 32 * k), smem_desc_rows<KB>(bbase + 32 * k), idesc, it > 0 || k > 0);
             umma_commit(smem_u32(&empty[s]));
             counts[1] = it + 1;
         }
@@ -239,7 +255,7 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
                      : "r"(taddr));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (!valid || py >= a.H || px >= a.W) continue;
-        store_row16(a.y + (((size_t)n * a.H + py) * a.W + px) * a.Cout, c0, a.Cout, v, s_bias, a.relu);
+        store_row16(a.y + (((size_t)n * a.H + py) * a.W + px) * a.Cout + co0, c0, a.Cout - co0, v, s_bias, a.relu);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -455,8 +471,9 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             unsigned char *gs = smem + s * a.stage_bytes + xall * WG_CHUNK;
             for (int q = threadIdx.x - 64; q < TC_BM * gunits; q += 64) {
                 const int r = q & (TC_BM - 1), U = q >> 7;
+                const int py = y0 + r / a.BW, px = x0 + r % a.BW;
                 *reinterpret_cast<uint4 *>(gs + (U >> 2) * WG_CHUNK + sw64_off(r, U & 3)) =
-                    pixel_unit(a.g, a.Cout, a.H, a.W, n, y0 + r / a.BW, x0 + r % a.BW, U);
+                    py < a.H && px < a.W ? pixel_unit(a.g, a.Cout, a.H, a.W, n, py, px, U) : make_uint4(0u, 0u, 0u, 0u);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
@@ -1189,8 +1206,8 @@ int *error_flag()
 
 }  // namespace
 
-// The tensor-core path covers Cin a multiple of 32, Cout <= 128, and images tiled exactly by
-// 128-pixel blocks (W a multiple of 128, or a power of two below it with H a multiple of 128 / W).
+// Whether 128-pixel blocks tile the image exactly (W a multiple of 128, or a power of two below it with
+// H a multiple of 128 / W): what the kernels whose threads write the im2col tiles need.
 static bool tiles_exactly(int H, int W)
 {
     if (H < 1 || W < 1) return false;
@@ -1199,15 +1216,32 @@ static bool tiles_exactly(int H, int W)
     return H % (TC_BM / W) == 0;
 }
 
-bool plbm_nn_tc_supported(int H, int W, int Cin, int Cout)
+// The TMA-fed kernels' 128-pixel tiles: the power-of-two width that needs the fewest for the image, the
+// widest of equals.  Pixels of a tile outside the image are loaded as zeros and not stored.  (Ragged
+// images took the mma.sync kernel, 100 us and more a layer: inference of 64 x 64 pixels, whose inner layers
+// have 32 x 32 to 4 x 4, 979 -> 154 us, of 128 x 128 527 -> 156.)
+struct ImageTiles { int BW, BH, x, y; };
+static ImageTiles image_tiles(int H, int W)
 {
-    if (Cin % TC_KB != 0 || Cin > 4096 || Cout < 1 || Cout > 128) return false;
-    return tiles_exactly(H, W);
+    ImageTiles best{};
+    for (int BW = TC_BM; BW >= 1; BW /= 2) {
+        const ImageTiles t{ BW, TC_BM / BW, (W + BW - 1) / BW, (H + TC_BM / BW - 1) / (TC_BM / BW) };
+        if (best.BW == 0 || (long long)t.x * t.y < (long long)best.x * best.y) best = t;
+    }
+    return best;
 }
 
-// y = act(conv3x3(x, w) + bias) on the tensor cores; x, y NHWC BF16; w [Cout][9][Cin] BF16.
+// The TMA-fed kernel covers Cin a multiple of 32, Cout <= 128.
+bool plbm_nn_tc_supported(int H, int W, int Cin, int Cout)
+{
+    return H >= 1 && W >= 1 && Cin % TC_KB == 0 && Cin >= TC_KB && Cin <= 4096 && Cout >= 1 && Cout <= 128;
+}
+
+// y = act(conv3x3(x, w) + bias) on the tensor cores; x, y NHWC BF16; w [Cout][9][Cin] BF16.  dgrad: w are
+// flipped weights and y an input gradient.  On ragged images its taps are then accumulated from the last to
+// the first, the order of the layer's own taps and of the mma.sync kernel's, which gives the same bits.
 int plbm_nn_tc_conv(const void *x, const void *w, const float *bias, void *y, int N, int H, int W, int Cin, int Cout,
-                    int relu, cudaStream_t s)
+                    int relu, bool dgrad, cudaStream_t s)
 {
     PFN_cuTensorMapEncodeTiled_v12000 enc = encode_fn();
     int *err = error_flag();
@@ -1217,34 +1251,32 @@ int plbm_nn_tc_conv(const void *x, const void *w, const float *bias, void *y, in
     {
         std::lock_guard<std::mutex> g(mu);
         if (!attr) {
-            if (cudaFuncSetAttribute(k_conv_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess)
+            if (cudaFuncSetAttribute(k_conv_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess ||
+                cudaFuncSetAttribute(k_conv_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess)
                 return PLBM_ERR_CUDA;
             attr = true;
         }
     }
-    const int BW = W >= TC_BM ? TC_BM : W, BH = TC_BM / BW;
-    const int npad = (Cout + 15) / 16 * 16;
+    const ImageTiles t = image_tiles(H, W);
+    const int BW = t.BW, BH = t.BH, npad = (Cout + 15) / 16 * 16;
+    // tensor maps of the K blocks: kb channels of 128 pixels, of npart output channels' weights
     CUtensorMap xmap, wmap;
-    {
-        const cuuint64_t dims[4] = { (cuuint64_t)Cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N };
-        const cuuint64_t strides[3] = { (cuuint64_t)Cin * 2, (cuuint64_t)W * Cin * 2, (cuuint64_t)H * W * Cin * 2 };
-        const cuuint32_t box[4] = { TC_KB, (cuuint32_t)BW, (cuuint32_t)BH, 1 };
+    auto maps = [&](int kb, int npart) {
+        const CUtensorMapSwizzle swizzle = kb == TC_KB ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
         const cuuint32_t es[4] = { 1, 1, 1, 1 };
-        if (enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(x), dims, strides, box, es,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return PLBM_ERR_ARGUMENT;
-    }
-    {
-        const cuuint64_t dims[3] = { (cuuint64_t)Cin, 9, (cuuint64_t)Cout };
-        const cuuint64_t strides[2] = { (cuuint64_t)Cin * 2, (cuuint64_t)9 * Cin * 2 };
-        const cuuint32_t box[3] = { TC_KB, 1, (cuuint32_t)npad };
-        const cuuint32_t es[3] = { 1, 1, 1 };
-        if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(w), dims, strides, box, es,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return PLBM_ERR_ARGUMENT;
-    }
+        const cuuint64_t xdims[4] = { (cuuint64_t)Cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N };
+        const cuuint64_t xstrides[3] = { (cuuint64_t)Cin * 2, (cuuint64_t)W * Cin * 2, (cuuint64_t)H * W * Cin * 2 };
+        const cuuint32_t xbox[4] = { (cuuint32_t)kb, (cuuint32_t)BW, (cuuint32_t)BH, 1 };
+        const cuuint64_t wdims[3] = { (cuuint64_t)Cin, 9, (cuuint64_t)Cout };
+        const cuuint64_t wstrides[2] = { (cuuint64_t)Cin * 2, (cuuint64_t)9 * Cin * 2 };
+        const cuuint32_t wbox[3] = { (cuuint32_t)kb, 1, (cuuint32_t)npart };
+        return enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(x), xdims, xstrides, xbox, es,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS &&
+               enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(w), wdims, wstrides, wbox, es,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
     // rows of 128 pixels: the halo-row kernel, when the layer's weights and two stages fit
     const int kblocks = Cin / TC_KB;
     const int w_bytes = 9 * kblocks * npad * 64;
@@ -1256,6 +1288,7 @@ int plbm_nn_tc_conv(const void *x, const void *w, const float *bias, void *y, in
     // each persistent CTA loads the whole layer's weights first: worth it from four tiles per SM on
     if (W % TC_BM == 0 && hstages >= 1 && N * H * (W / TC_BM) >= 4 * sms) {
         CUtensorMap hmap;
+        if (!maps(TC_KB, npad)) return PLBM_ERR_ARGUMENT;
         const cuuint64_t dims[4] = { (cuuint64_t)Cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N };
         const cuuint64_t strides[3] = { (cuuint64_t)Cin * 2, (cuuint64_t)W * Cin * 2, (cuuint64_t)H * W * Cin * 2 };
         const cuuint32_t box[4] = { TC_KB, HALO_ROW, 1, 1 };
@@ -1279,17 +1312,29 @@ int plbm_nn_tc_conv(const void *x, const void *w, const float *bias, void *y, in
         return nn_launch(k_conv_halo_tc, (unsigned)(h.tiles < sms ? h.tiles : sms), 224, smem, s, hmap, wmap, h) == cudaSuccess
                    ? PLBM_OK : PLBM_ERR_CUDA;
     }
-    // stages sized by the padded output channels, so narrow layers fit more CTAs per SM
-    const int stage = TC_A_BYTES + (npad * TC_KB * 2 + 1023) / 1024 * 1024;
-    const int tiles = N * (W / BW) * (H / BH);
+    const int tiles = N * t.x * t.y;
+    // Output channels are split over CTAs (at least 32 each) while those still fit one to an SM, and rows
+    // of 64 channels halve the rows TMA fetches, where Cin allows: a layer of few tiles waits for its
+    // loads.  1 x 256^2 inference, measured with one kernel for both row lengths: neither 234 us, split 227,
+    // longer rows 203, both 195 (and 176 with a kernel for each); 16 x 256^2, with tiles for several CTAs an
+    // SM, 665 / 636 without and with the longer rows.  Each value keeps its order of accumulation.
+    int parts = 1;
+    for (int p = 2; p <= npad / 32 && tiles * p <= sms; ++p)
+        if (npad % (16 * p) == 0) parts = p;
+    const int kb = Cin % 64 == 0 ? 64 : TC_KB;
+    const int npart = npad / parts, ctas = tiles * parts;
+    // stages sized by the CTA's output channels, so narrow layers fit more CTAs per SM
+    const int stage = TC_BM * kb * 2 + (npart * kb * 2 + 1023) / 1024 * 1024;
     // four stages let four CTAs share an SM; a layer with fewer tiles than SMs waits for its own loads
     // instead and takes all that fit (16 x 16 pixels, 128 -> 128 channels: 36 stages' worth of loads; a
     // 1 x 256^2 inference 215 -> 210 us, a 5 x 256^2 one 318 -> 309)
     const int fit = (TC_SMEM - 1024 - 256) / stage, most = fit < TC_MAX_STAGES ? fit : TC_MAX_STAGES;
-    const int stages = tiles <= sms ? most : tiles <= 2 * sms ? (most + 1) / 2 : TC_STAGES;
-    TcArgs a{ (__nv_bfloat16 *)y, bias, N, H, W, Cin, Cout, npad, relu, BW, BH, W / BW, H / BH, stage, stages, err };
-    return nn_launch(k_conv_tc, (unsigned)tiles, 128, (size_t)stages * stage + 1024 + 256, s, xmap, wmap, a) == cudaSuccess
-               ? PLBM_OK : PLBM_ERR_CUDA;
+    const int stages = ctas <= sms ? most : ctas <= 2 * sms ? (most + 1) / 2 : TC_STAGES * TC_KB / kb;
+    if (!maps(kb, npart)) return PLBM_ERR_ARGUMENT;
+    TcArgs a{ (__nv_bfloat16 *)y, bias, N, H, W, Cin, Cout, npart, relu, BW, BH, t.x, t.y, stage, stages,
+              dgrad && !tiles_exactly(H, W), err };
+    return nn_launch(kb == 64 ? k_conv_tc<64> : k_conv_tc<32>, dim3((unsigned)tiles, (unsigned)parts), 128,
+                     (size_t)stages * stage + 1024 + 256, s, xmap, wmap, a) == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
 }
 
 // The weight gradient runs on the TMA-fed tensor-core kernel for Cin a multiple of 32 up to 128,
@@ -1297,8 +1342,7 @@ int plbm_nn_tc_conv(const void *x, const void *w, const float *bias, void *y, in
 // image tilings of the forward kernel.
 bool plbm_nn_tc_wgrad_supported(int H, int W, int Cin, int Cout)
 {
-    if (Cin % TC_KB != 0 || Cin < TC_KB || Cin > 128 || Cout < 1 || Cout > WG_M) return false;
-    return tiles_exactly(H, W);
+    return H >= 1 && W >= 1 && Cin % TC_KB == 0 && Cin >= TC_KB && Cin <= 128 && Cout >= 1 && Cout <= WG_M;
 }
 
 // gw[co][tap][ci] += sum_p g[p][co] x[p + tap][ci] on the tensor cores (x, g NHWC BF16, gw FP32); with
@@ -1366,7 +1410,8 @@ int plbm_nn_tc_wgrad(const void *x, const void *g, float *gw, float *gb, int N, 
     WgArgs a{};
     a.gw = gw; a.g = (const __nv_bfloat16 *)g;
     a.N = N; a.H = H; a.W = W; a.Cin = Cin; a.Cout = Cout;
-    a.BW = W >= TC_BM ? TC_BM : W; a.BH = TC_BM / a.BW; a.tiles_x = W / a.BW; a.tiles_y = H / a.BH;
+    const ImageTiles t = image_tiles(H, W);
+    a.BW = t.BW; a.BH = t.BH; a.tiles_x = t.x; a.tiles_y = t.y;
     const int kbx = Cin / TC_KB;
     a.ntaps = kbx == 1 ? 9 : 3;                    // the TMEM columns of a CTA stay <= 384
     a.tg = a.ntaps * kbx <= 9 ? a.ntaps : 1;       // at most nine input tiles (72 KB) per stage
