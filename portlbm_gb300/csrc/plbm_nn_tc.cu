@@ -749,6 +749,36 @@ __device__ __forceinline__ uint4 im2col_unit(const __nv_bfloat16 *src, int C, in
     return make_uint4(v[0], v[1], v[2], v[3]);
 }
 
+// The im2col row of pixel (n, py, px) for C = 3 or 4 channels (the fields and the input of the operator), its
+// 9 C columns as CHUNKS * 16 words of two: the taps are compile-time, so no unit computes where its columns lie.
+template <int C, int CHUNKS>
+__device__ __forceinline__ void im2col_row(const __nv_bfloat16 *src, int H, int W, int n, int py, int px,
+                                           uint32_t (&v)[CHUNKS * 16])
+{
+#pragma unroll
+    for (int i = 0; i < CHUNKS * 16; ++i) v[i] = 0u;
+    const bool above = py > 0, below = py + 1 < H, left = px > 0, right = px + 1 < W;
+    const __nv_bfloat16 *centre = src + (((size_t)n * H + py) * W + px) * C;
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap) {
+        const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+        if ((dy >= 0 || above) && (dy <= 0 || below) && (dx >= 0 || left) && (dx <= 0 || right)) {
+            const __nv_bfloat16 *p = centre + ((long long)dy * W + dx) * C;
+            if constexpr (C == 4) {
+                const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p));
+                v[2 * tap] = q.x;
+                v[2 * tap + 1] = q.y;
+            } else {
+#pragma unroll
+                for (int ch = 0; ch < C; ++ch) {
+                    const int c = tap * C + ch;
+                    v[c >> 1] |= (uint32_t)ld_bf16_bits(p + ch) << (16 * (c & 1));
+                }
+            }
+        }
+    }
+}
+
 struct SmallArgs {
     const __nv_bfloat16 *x;     // forward: input [N,H,W,Cin]; weight gradient: input
     const __nv_bfloat16 *w;     // forward: weights [Cout][9 * Cin]
@@ -764,19 +794,23 @@ struct SmallArgs {
     int *err;
 };
 
-// Forward convolution of a narrow input: one 128-pixel tile per CTA; the threads write the im2col
-// tile (K-major: row = pixel, kchunks chunks of 32 columns) and the weights (row = output channel),
-// one thread issues kchunks * 2 MMAs (K = 16 each) into a TMEM accumulator of npad columns.
-__global__ void __launch_bounds__(SM_BUILD, 8) k_conv_small_tc(SmallArgs a)
+// Forward convolution of a narrow input: the threads write a 128-pixel tile's im2col rows (K-major:
+// row = pixel, kchunks chunks of 32 columns) and, once, the weights (row = output channel); one thread
+// issues kchunks * 2 MMAs (K = 16 each) into a TMEM accumulator of npad columns.  A tile is a chain of
+// latencies (loads, MMAs, accumulator, stores), so several CTAs share an SM, each walks every gridDim.x-th
+// tile, and the next tile's rows are written to a second buffer while the MMAs of this one run.
+// (A CTA of its own for every tile, with its set-up and weights: 16 x 256^2, 4 -> 32 channels, 54 -> 45 us;
+// the head's input gradient, 3 -> 32, 89 -> 36 us; with the taps of im2col_row computed per unit 60 and 94.)
+__global__ void __launch_bounds__(SM_BUILD, 6) k_conv_small_tc(SmallArgs a)
 {
     __shared__ float s_bias[128];
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
     unsigned char *smem = tc_smem_raw + ((1024 - (smem_u32(tc_smem_raw) & 1023)) & 1023);
-    unsigned char *As = smem, *Bs = smem + a.kchunks * WG_CHUNK;
+    unsigned char *As = smem, *Bs = smem + 2 * a.kchunks * WG_CHUNK;
     unsigned long long *done = reinterpret_cast<unsigned long long *>(Bs + a.kchunks * a.npad * 64);
     unsigned *tmem_slot = reinterpret_cast<unsigned *>(done + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
     const unsigned ncols = a.npad <= 32 ? 32u : (a.npad <= 64 ? 64u : 128u);
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(done), 1);
@@ -790,18 +824,42 @@ __global__ void __launch_bounds__(SM_BUILD, 8) k_conv_small_tc(SmallArgs a)
     nn_begin();
     stage_bias(s_bias, a.bias, a.Cout, a.npad);
     const int per_img = a.tiles_x * a.tiles_y;
-    const int n = blockIdx.x / per_img, t2 = blockIdx.x % per_img;
-    const int y0 = (t2 / a.tiles_x) * a.BH, x0 = (t2 % a.tiles_x) * a.BW;
-    {   // A: thread r writes row r (pixel r of the tile)
-        const int r = threadIdx.x, px = x0 + r % a.BW, py = y0 + r / a.BW;
+    const int row = threadIdx.x, ry = row / a.BW, rx = row % a.BW;   // the thread's pixel of each tile
+    auto origin = [&](int tile, int &n, int &py, int &px) {
+        n = tile / per_img;
+        const int t = tile % per_img, ty = t / a.tiles_x;
+        py = ty * a.BH + ry;
+        px = (t - ty * a.tiles_x) * a.BW + rx;
+    };
+    auto build = [&](int tile, unsigned char *to) {   // A: the thread writes its pixel's row
+        int n, py, px;
+        origin(tile, n, py, px);
+        auto store = [&](const auto &v) {
+#pragma unroll
+            for (int k = 0; k < (int)(sizeof(v) / 16); ++k)
+                *reinterpret_cast<uint4 *>(to + (k >> 2) * WG_CHUNK + sw64_off(row, k & 3)) =
+                    make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        };
+        if (a.Cin == 4) {
+            uint32_t v[32];
+            im2col_row<4, 2>(a.x, a.H, a.W, n, py, px, v);
+            return store(v);
+        }
+        if (a.Cin == 3) {
+            uint32_t v[16];
+            im2col_row<3, 1>(a.x, a.H, a.W, n, py, px, v);
+            return store(v);
+        }
         for (int c = 0; c < a.kchunks; ++c) {
             uint4 u[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) u[k] = im2col_unit(a.x, a.Cin, a.H, a.W, n, py, px, c * 4 + k);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4 *>(As + c * WG_CHUNK + sw64_off(r, k)) = u[k];
+            for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4 *>(to + c * WG_CHUNK + sw64_off(row, k)) = u[k];
         }
-    }
+    };
+    int tile = blockIdx.x;
+    build(tile, As);
     const int K = 9 * a.Cin;
     for (int i = threadIdx.x; i < a.kchunks * a.npad * 4; i += SM_BUILD) {   // B: row j = output channel j
         const int c = i / (a.npad * 4), rem = i - c * a.npad * 4, j = rem >> 2, k = rem & 3;
@@ -815,46 +873,54 @@ __global__ void __launch_bounds__(SM_BUILD, 8) k_conv_small_tc(SmallArgs a)
         }
         *reinterpret_cast<uint4 *>(Bs + c * a.npad * 64 + sw64_off(j, k)) = make_uint4(v[0], v[1], v[2], v[3]);
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tiles are read by the tensor cores
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const unsigned tmem = *tmem_slot;
-    if (threadIdx.x == 0) {
-        const unsigned idesc = instr_desc(a.npad);
-        const unsigned abase = smem_u32(As), bbase = smem_u32(Bs);
-        for (int c = 0; c < a.kchunks; ++c)
+    unsigned tmem = 0, parity = 0;
+    bool valid = true;
+    for (int stage = 0; tile < a.total_tiles; stage ^= 1, parity ^= 1u) {
+        unsigned char *from = As + stage * a.kchunks * WG_CHUNK;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tiles are read by the tensor cores
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (!__syncthreads_and(valid)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem = *tmem_slot;
+        if (threadIdx.x == 0) {
+            const unsigned idesc = instr_desc(a.npad);
+            const unsigned abase = smem_u32(from), bbase = smem_u32(Bs);
+            for (int c = 0; c < a.kchunks; ++c)
 #pragma unroll
-            for (int k = 0; k < 2; ++k)
-                umma(tmem, smem_desc_sw64(abase + c * WG_CHUNK + 32 * k), smem_desc_sw64(bbase + c * a.npad * 64 + 32 * k),
-                     idesc, c > 0 || k > 0);
-        umma_commit(smem_u32(done));
-    }
-    const bool valid = mbar_wait(smem_u32(done), 0);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int row = warp * 32 + lane;
-    const int px = x0 + row % a.BW, py = y0 + row / a.BW;
-    for (int c0 = 0; c0 < a.npad; c0 += 16) {
-        unsigned v[16];
-        const unsigned taddr = tmem + ((unsigned)(warp * 32) << 16) + (unsigned)c0;
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                       "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                     : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (!valid || py >= a.H || px >= a.W) continue;
-        store_row16(a.y + (((size_t)n * a.H + py) * a.W + px) * a.Cout, c0, a.Cout, v, s_bias, a.relu);
+                for (int k = 0; k < 2; ++k)
+                    umma(tmem, smem_desc_sw64(abase + c * WG_CHUNK + 32 * k),
+                         smem_desc_sw64(bbase + c * a.npad * 64 + 32 * k), idesc, c > 0 || k > 0);
+            umma_commit(smem_u32(done));
+        }
+        __syncwarp();
+        int n, py, px;
+        origin(tile, n, py, px);
+        tile += gridDim.x;
+        if (tile < a.total_tiles) build(tile, As + (stage ^ 1) * a.kchunks * WG_CHUNK);
+        valid = mbar_wait(smem_u32(done), parity);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        __syncwarp();
+        for (int c0 = 0; c0 < a.npad; c0 += 16) {
+            unsigned v[16];
+            const unsigned taddr = tmem + ((unsigned)(warp * 32) << 16) + (unsigned)c0;
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                           "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                         : "r"(taddr));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (valid) store_row16(a.y + (((size_t)n * a.H + py) * a.W + px) * a.Cout, c0, a.Cout, v, s_bias, a.relu);
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (threadIdx.x == 0 && !valid) {
+    const bool ok = __syncthreads_and(valid);
+    if (threadIdx.x == 0 && !ok) {   // the MMAs issued complete, bounded, before the TMEM is released
         atomicExch(a.err, 1);
-        mbar_wait(smem_u32(done), 0);
+        mbar_wait(smem_u32(done), parity ^ 1u);
     }
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*tmem_slot), "r"(ncols) : "memory");
     }
 }
 
@@ -1482,9 +1548,13 @@ int plbm_nn_tc_small_conv(const void *x, const void *w, const float *bias, void 
     a.BW = W >= TC_BM ? TC_BM : W; a.BH = TC_BM / a.BW; a.tiles_x = W / a.BW; a.tiles_y = H / a.BH;
     a.kchunks = (9 * Cin + TC_KB - 1) / TC_KB;
     a.err = err;
-    const int smem = a.kchunks * (WG_CHUNK + a.npad * 64) + 1024 + 64;
-    return nn_launch(k_conv_small_tc, (unsigned)(N * a.tiles_x * a.tiles_y), SM_BUILD, smem, s, a) == cudaSuccess ? PLBM_OK
-                                                                                                                : PLBM_ERR_CUDA;
+    const int smem = a.kchunks * (2 * WG_CHUNK + a.npad * 64) + 1024 + 64;   // at most 42 KB
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
+    a.total_tiles = N * a.tiles_x * a.tiles_y;
+    const int ctas = sms * 6;   // six share an SM (38 KB each at 4 -> 32 channels); fewer tiles: one each
+    return nn_launch(k_conv_small_tc, (unsigned)(a.total_tiles < ctas ? a.total_tiles : ctas), SM_BUILD, smem, s, a) ==
+                   cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
 }
 
 // Weight gradient of a layer with Cin <= 32 (its 9 * Cin (tap, ci) columns in at most 9 chunks of 32)

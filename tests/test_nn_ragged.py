@@ -79,3 +79,26 @@ def test_ragged_convolution_and_gradients(plbm, n, h, w, cin, cout):
     close(gb.double().cpu().numpy(), want_b, size_b, n * h * w, rounded=False)
     failed = ctypes.c_int(1)
     assert lib.plbm_nn_status(ctypes.byref(failed)) == 0 and failed.value == 0
+
+
+@pytest.mark.parametrize("n,h,w,cin,cout", [(5, 256, 128, 4, 32), (5, 256, 128, 3, 12), (4, 512, 64, 7, 5), (1, 2, 64, 3, 64),
+                                           (3, 4, 256, 4, 3)])
+def test_narrow_layers_of_many_and_few_tiles(plbm, n, h, w, cin, cout):
+    """The kernel whose threads write the im2col rows, with more tiles than CTAs share the GPU and with few."""
+    from portlbm_gb300 import warmstart as ws
+    lib = ws._fns()
+    assert lib.plbm_nn_conv_on_tensor_cores(h, w, cin, cout) == 1
+    rng = np.random.default_rng(h + cin)
+    x = nn_ref.bf16_round(rng.standard_normal((n, h, w, cin)))
+    wt = nn_ref.bf16_round(rng.standard_normal((cout, 9 * cin)) / np.sqrt(9 * cin))
+    b = rng.standard_normal(cout).astype(np.float32)
+    xd, wd, bd = bf(x), bf(wt), torch.tensor(b).cuda()
+    size = n * h * w * cout
+    y = torch.full((size + 4096,), 7.0, dtype=torch.bfloat16, device="cuda")
+    assert lib.plbm_nn_conv_fwd(xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), y.data_ptr(), n, h, w, cin, cout, 0, None) == 0
+    want = nn_ref.conv_fwd(x, wt, b.astype(np.float64), False)
+    bound = 2.0 ** -8 * np.abs(want) + (9 * cin + 2) * 2.0 ** -24 * nn_ref.conv_fwd(np.abs(x), np.abs(wt), np.abs(b).astype(np.float64))
+    assert (np.abs(host(y[:size]).reshape(n, h, w, cout) - want) <= bound).all()
+    assert (y[size:] == 7.0).all()
+    failed = ctypes.c_int(1)
+    assert lib.plbm_nn_status(ctypes.byref(failed)) == 0 and failed.value == 0
