@@ -5,11 +5,16 @@
 
 namespace plbm {
 
+unsigned two_step_blocks(int W)
+{
+    const int strips = (W + PAIR_COLUMNS - 1) / PAIR_COLUMNS;
+    return (unsigned)((strips + PAIR_WARPS - 1) / PAIR_WARPS);
+}
+
 template <int PREC, int L>
 static cudaError_t launch(const StepParams &p, int rows, cudaStream_t s)
 {
-    const int strips = (p.W + PAIR_COLUMNS - 1) / PAIR_COLUMNS;
-    const dim3 grid((unsigned)((strips + PAIR_WARPS - 1) / PAIR_WARPS), (unsigned)((p.H + rows - 1) / rows));
+    const dim3 grid(two_step_blocks(p.W), (unsigned)((p.H + rows - 1) / rows));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(32, PAIR_WARPS);

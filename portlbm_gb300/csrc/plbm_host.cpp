@@ -871,7 +871,7 @@ struct plbm_handler {
         }
     }
 
-    // The kernels of nptl and lptl that pay on domains whose two lattices outgrow L2:
+    // The kernels of nptl and lptl that pay on domains whose two lattices outgrow L2, or that are small:
     //  * plain steps two a launch.  Shifted forms from half of L2 on: f32 72 MB of lattices 10.7 us a step
     //    singly against 10.5, 111 MB 19.4 / 14.6, 216 MB 38.1 / 27.0; f16s 72 MB 20.6 / 19.5, 108 MB
     //    36.3 / 27.3; below (1000 x 300) 4.6 / 5.4.  F64_Q60, bound by instructions as much as by HBM,
@@ -879,6 +879,11 @@ struct plbm_handler {
     //    a strip trade rows done twice against blocks enough for every SM: shifted 4 up to 4 M nodes
     //    (3 M: 27.0, with 8 rows 28.0), 8 up to 32 M (8 M: 59.9, with 4 rows 61.6), 16 above (67 M: 429,
     //    with 8 rows 445); Q60 16 up to 16 M, 32 above (67 M: 1222, with 16 rows 1254).
+    //    Shifted forms also up to 2^16 nodes, a row a strip: a step there is the latency of a launch, and of
+    //    two steps a launch only the second collision adds to it (400 x 100: f32 2.98 / 2.24 us, f16s 3.46 /
+    //    2.57, f16c 3.5 / 3.2; 62 x 30: 2.75 / 2.12; 320 x 200: 2.99 / 2.37; but 512 x 320 3.71 / 3.90: every
+    //    row's first step is done three times), where the blocks (four strips of 30 columns) are one wave, as
+    //    those of a tall narrow domain are not (31 x 2000: 4.5 / 4.7, 8 x 4000: 4.9 / 6.0).  Q60's collision is too long for that (400 x 100: 3.2 / 4.0).
     //  * nptl's 2-byte forms step vectorised rows in the stream layout from four fifths of L2 on; on
     //    smaller domains, where the few warps of 256 nodes wait, the scalar kernel (1000 x 300 f16s 9.3
     //    against 6.0 us, 2000 x 500 14.3 / 11.3, 3000 x 1000 32.8 / 34.1).
@@ -891,6 +896,9 @@ struct plbm_handler {
         vec_rows = lattices > cache / 5 * 4;
         pair_rows = 0;
         if (!two_lattice() || debug) return;
+        int sms = 0;
+        cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opt.device), "device attribute");
+        if (shifted && N <= (1ull << 16) && (unsigned long long)plbm::two_step_blocks(W) * H <= 8ull * sms) pair_rows = 1;
         if (shifted && lattices > cache / 2) pair_rows = N < (1ull << 22) ? 4 : N < (1ull << 25) ? 8 : 16;
         if (prec == PLBM_F64_Q60 && lattices > 8 * cache) pair_rows = N < (1ull << 24) ? 16 : 32;
         // the kernel's offsets (bytes, values of 8-byte storage) and its grid height are 32 and 16 bits

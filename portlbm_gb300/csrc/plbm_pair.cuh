@@ -1,5 +1,6 @@
 // plbm_pair.cuh — two timesteps of the two-lattice algorithms in one pass over memory, for the shifted
-// forms (FP32 arithmetic) and F64_Q60, whose single steps of a large domain are bound by HBM.
+// forms (FP32 arithmetic) and F64_Q60, whose single steps of a large domain are bound by HBM and of a
+// small one by the latency of a launch.
 //
 // A warp owns a strip of 30 columns and marches up `rows` rows of it.  At row r it pulls the first step's
 // populations of its 32 columns from memory (the outermost two only feed their neighbours), collides

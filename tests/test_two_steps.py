@@ -1,4 +1,4 @@
-"""Two-step launches of nptl and lptl (csrc/plbm_pair.cuh, domains whose lattices exceed L2) against
+"""Two-step launches of nptl and lptl (csrc/plbm_pair.cuh, domains whose lattices exceed L2 and small ones) against
 single steps of the same handler: the same values, whatever the domain's remainders of a strip's
 columns and rows, the number of steps, the gather and the layout."""
 import numpy as np
@@ -9,7 +9,10 @@ pytestmark = pytest.mark.gpu
 
 def handler(plbm, alg, lay, precision, w, h, porous, rho_in=1.03):
     props = plbm.Properties(alg, lay, False, 1024, 10 ** 6, 10 ** 6, "circle", h, w, 0.0, 0.0, rho_in, 0.0, 0.0, 1.0, 0.6)
-    mask = plbm.porous_disks(w, h, 5, 0.75) if porous else None
+    mask = None
+    if porous:   # disks need room; small domains take single solid nodes
+        small = min(w, h) < 64
+        mask = (np.random.default_rng(w * h).random((h, w)) < 0.2).astype(np.int8) if small else plbm.porous_disks(w, h, 5, 0.75)
     return plbm.create_handler(props, precision=precision, mask=mask)
 
 
@@ -18,10 +21,17 @@ def fields(hd):
     return [hd.get_densities(), hd.get_x_velocities(), hd.get_y_velocities(), hd.get_absolute_velocities()]
 
 
-# two-step launches are taken from 0.5 (shifted forms) and 8 (f64_q60) times L2's 129 MB of lattices on
+# two-step launches are taken from 0.5 (shifted forms) and 8 (f64_q60) times L2's 129 MB of lattices on, and
+# up to 65536 nodes (row pitch included) by the shifted forms
 SIZES = {"f32": [(1603, 1153), (31, 60001), (60, 30011), (2501, 1801)],
          "f16s": [(2401, 1511), (61, 60007), (2130, 2011)], "bf16s": [(2401, 1511)], "f16c": [(2431, 1517)],
          "f64_q60": [(3031, 2507), (4111, 4093)]}
+SMALL = [(2, 2), (2, 9), (3, 5), (4, 3), (29, 4), (30, 31), (31, 7), (32, 64), (33, 20), (61, 100), (62, 30), (512, 128),
+         (1003, 63), (513, 128)]
+SIZES["f32"] += SMALL
+SIZES["f16s"] += SMALL
+SIZES["bf16s"] += SMALL[2::4]
+SIZES["f16c"] += SMALL[3::4]
 CASES = [(p, w, h) for p, sizes in SIZES.items() for w, h in sizes]
 
 
@@ -76,7 +86,8 @@ def test_frames_and_precision_change(plbm):
 
 
 @pytest.mark.parametrize("precision,w,h,pairs", [("f16s", 2401, 1511, True), ("f64_q60", 3031, 2507, True),
-                                                 ("f64_q60", 400, 100, False), ("f64_strict", 400, 100, False)])
+                                                 ("f64_q60", 400, 100, False), ("f64_strict", 400, 100, False),
+                                                 ("f32", 400, 100, True), ("f32", 512, 129, False)])
 def test_launch_accounting(plbm, precision, w, h, pairs):
     """run_launches follows the schedule: an odd first step, four plain steps in two launches, the rest
     and the result step one by one."""
