@@ -8,8 +8,8 @@
 // rounded once to nearest, ties to even.  What stays on the FP64 pipe (25 operations) are the
 // products of two variables and the last relaxation step, whose operands have no common scale.
 //
-// Measured (k_nptl<F64_STRICT, STREAM>, 4096 x 4096): 5.7 k -> 18.9 k MLUPS; 2000 x 500: npol records
-// 194 -> 74.4 us a step, nsol stream 194 -> 64.5 us.  With 25 FP64 instructions and about 780 on the ALU pipe
+// Measured (k_nptl<F64_STRICT, STREAM>, 4096 x 4096): 5.7 k -> 17.8 k MLUPS; 2000 x 500: npol records
+// 194 -> 72.4 us a step, nsol stream 194 -> 62.1 us.  With 25 FP64 instructions and about 780 on the ALU pipe
 // a warp both pipes are 70 % busy (the plain sequence keeps the FP64 pipe full); each further
 // operation moved off the FP64 pipe costs 12 to 30 ALU instructions against its 32 ALU slots' time.
 // Converting |j| with I2F.F64 instead of by hand: 16.2 k; 4.5 a and 1.5 u^2 as FP64 products: 17.7 k.
