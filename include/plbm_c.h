@@ -191,8 +191,9 @@ int plbm_benchmark_run(const char *settings_path, const char *benchmark_path, co
 int plbm_benchmark_work_group_sizes(unsigned max_work_group_size, unsigned *out, unsigned capacity, unsigned *count);
 /* Kernel launches of one step that writes results (for launch accounting). */
 int plbm_launches_per_step(plbm_handler *h, unsigned *n);
-/* Kernel launches the next plbm_run_steps(h, n) issues: plain steps (no results) run two a launch
- * on large nptl / lptl domains of the shifted forms and of the Q60 form, and on small ones of the shifted forms. */
+/* Kernel launches the next plbm_run_steps(h, n) issues: plain steps (no results) of nptl and lptl run
+ * two a launch on large domains of the shifted forms and of the Q60 form, and on small domains and
+ * porous records of the shifted forms. */
 int plbm_run_launches(plbm_handler *h, unsigned n, unsigned *launches);
 /* Algorithmic HBM bytes per node update of the hot kernel (9 loads + 9 stores). */
 int plbm_bytes_per_node(plbm_handler *h, double *bytes);

@@ -883,7 +883,13 @@ struct plbm_handler {
     //    two steps a launch only the second collision adds to it (400 x 100: f32 2.98 / 2.24 us, f16s 3.46 /
     //    2.57, f16c 3.5 / 3.2; 62 x 30: 2.75 / 2.12; 320 x 200: 2.99 / 2.37; but 512 x 320 3.71 / 3.90: every
     //    row's first step is done three times), where the blocks (four strips of 30 columns) are one wave, as
-    //    those of a tall narrow domain are not (31 x 2000: 4.5 / 4.7, 8 x 4000: 4.9 / 6.0).  Q60's collision is too long for that (400 x 100: 3.2 / 4.0).
+    //    those of a tall narrow domain are not (31 x 2000: 4.5 / 4.7, 8 x 4000: 4.9 / 6.0).  Q60's collision
+    //    is too long for that (400 x 100: 3.2 / 4.0).
+    //    And shifted records of porous domains at any size, two rows a strip: a single step's warps that hold
+    //    a solid node, most of them, store their records value by value (512 x 256: f32 4.64 / 3.51, f16s
+    //    5.25 / 3.89; 700 x 300: f32 6.05 / 4.01, f16s 6.84 / 4.56, f16c 6.67 / 5.71; 1000 x 800: 13.1 / 9.8,
+    //    14.7 / 10.5, 16.3 / 14.6; but in an open channel 1024 x 512 f32 7.44 / 8.54, and f16c with few
+    //    strips, 64 x 3000, 8.1 / 8.4).
     //  * nptl's 2-byte forms step vectorised rows in the stream layout from four fifths of L2 on; on
     //    smaller domains, where the few warps of 256 nodes wait, the scalar kernel (1000 x 300 f16s 9.3
     //    against 6.0 us, 2000 x 500 14.3 / 11.3, 3000 x 1000 32.8 / 34.1).
@@ -899,6 +905,7 @@ struct plbm_handler {
         int sms = 0;
         cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opt.device), "device attribute");
         if (shifted && N <= (1ull << 16) && (unsigned long long)plbm::two_step_blocks(W) * H <= 8ull * sms) pair_rows = 1;
+        if (shifted && porous && lay == plbm::COLLISION && !pair_rows && (prec != PLBM_F16C || W >= 256)) pair_rows = 2;
         if (shifted && lattices > cache / 2) pair_rows = N < (1ull << 22) ? 4 : N < (1ull << 25) ? 8 : 16;
         if (prec == PLBM_F64_Q60 && lattices > 8 * cache) pair_rows = N < (1ull << 24) ? 16 : 32;
         // the kernel's offsets (bytes, values of 8-byte storage) and its grid height are 32 and 16 bits

@@ -28,6 +28,9 @@ SIZES = {"f32": [(1603, 1153), (31, 60001), (60, 30011), (2501, 1801)],
          "f64_q60": [(3031, 2507), (4111, 4093)]}
 SMALL = [(2, 2), (2, 9), (3, 5), (4, 3), (29, 4), (30, 31), (31, 7), (32, 64), (33, 20), (61, 100), (62, 30), (512, 128),
          (1003, 63), (513, 128)]
+MIDDLE = [(353, 257), (1003, 401)]       # two steps a launch in porous records, single steps elsewhere
+for form in ("f32", "f16s", "bf16s", "f16c"):
+    SIZES[form] += MIDDLE
 SIZES["f32"] += SMALL
 SIZES["f16s"] += SMALL
 SIZES["bf16s"] += SMALL[2::4]
