@@ -331,6 +331,9 @@ int plbm_nn_relu_bwd_bias(const void *y, void *g, float *gb, long long P, int C,
 enum { PLBM_NN_GRAD = 0, PLBM_NN_GRAD_UP2 = 1, PLBM_NN_GRAD_POOL2 = 2 };
 int plbm_nn_relu_bwd_bias_from(int from, const void *g, const void *skip, const void *y, void *out, float *gb, int N, int H,
                                int W, int C, void *stream);
+/* 2x2 average pooling to [N,H/2,W/2,C] and nearest up-sampling from [N,H/2,W/2,C] (H and W even, otherwise
+ * PLBM_ERR_ARGUMENT), with their backward passes; the last row or column of an odd extent is not pooled, and
+ * its gradient is zero. */
 int plbm_nn_pool2(const void *x, void *y, int N, int H, int W, int C, void *stream);
 int plbm_nn_pool2_bwd(const void *gy, void *gx, int N, int H, int W, int C, void *stream);
 int plbm_nn_up2(const void *x, void *y, int N, int H, int W, int C, void *stream);
@@ -343,7 +346,8 @@ int plbm_nn_assemble_host(const int8_t *mask, const float *features, void *y, in
  * 2x2 average pooling; back up per level nearest upsampling, a convolution, the skip addition of the
  * level's encoder output and a convolution; the head.  layers: 2 levels + 2 (levels - 1) + 1 of them in
  * that order.  acts: the device buffers the results go to, in the order they are computed (each layer's,
- * pooling's, upsampling's and addition's). */
+ * pooling's, upsampling's and addition's).  H and W are multiples of 2^(levels - 1): PLBM_ERR_ARGUMENT
+ * otherwise. */
 typedef struct {
     const void *w;
     const float *bias;

@@ -217,7 +217,10 @@ __global__ void k_pool2_bwd(const __nv_bfloat16 *gy, __nv_bfloat16 *gx, int N, i
         const int x = (int)(t % W); t /= W;
         const int yv = (int)(t % H);
         const int n = (int)(t / H);
-        gx[i] = __float2bfloat16_rn(0.25f * __bfloat162float(gy[(((size_t)n * Ho + yv / 2) * Wo + x / 2) * C + c]));
+        // an odd extent's last row or column belongs to no pooled pixel
+        const bool pooled = yv / 2 < Ho && x / 2 < Wo;
+        gx[i] = __float2bfloat16_rn(pooled ? 0.25f * __bfloat162float(gy[(((size_t)n * Ho + yv / 2) * Wo + x / 2) * C + c])
+                                           : 0.0f);
     }
 }
 
@@ -477,7 +480,8 @@ __global__ void k_pool2_v(const uint4 *x, uint4 *y, unsigned N, unsigned H, unsi
     }
 }
 
-// Unit cu of input-gradient pixel p of [N][H][W][CU] (H, W the input size): a quarter of its pooled unit.
+// Unit cu of input-gradient pixel p of [N][H][W][CU] (H, W the input size): a quarter of its pooled unit.  Not
+// for the last row or column of an odd extent, which has none.
 __device__ __forceinline__ uint4 pool2_bwd_unit(const uint4 *gy, unsigned p, unsigned cu, unsigned H, unsigned W, unsigned CU)
 {
     const unsigned x = p % W, t2 = p / W, yv = t2 % H, n = t2 / H;
@@ -491,8 +495,10 @@ __device__ __forceinline__ uint4 pool2_bwd_unit(const uint4 *gy, unsigned p, uns
 __global__ void k_pool2_bwd_v(const uint4 *gy, uint4 *gx, unsigned N, unsigned H, unsigned W, unsigned CU)
 {
     const unsigned total = N * H * W * CU;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
-        gx[i] = pool2_bwd_unit(gy, i / CU, i % CU, H, W, CU);
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const unsigned p = i / CU, x = p % W, y = p / W % H;
+        gx[i] = y / 2 < H / 2 && x / 2 < W / 2 ? pool2_bwd_unit(gy, p, i % CU, H, W, CU) : make_uint4(0u, 0u, 0u, 0u);
+    }
 }
 
 // gb[c] += sum over the P pixels of a gradient: thread (pixel lane q, unit u) of a block of
@@ -823,6 +829,8 @@ int plbm_nn_pool2_bwd(const void *gy, void *gx, int N, int H, int W, int C, void
 
 int plbm_nn_up2(const void *x, void *y, int N, int H, int W, int C, void *stream)
 {
+    // an odd output extent's last row or column has no input pixel
+    if (N < 1 || H < 1 || W < 1 || C < 1 || H % 2 || W % 2) return PLBM_ERR_ARGUMENT;
     if (vec8(C, (long long)N * H * W * C, x, y)) {
         return launched(nn_launch(k_up2_v, (unsigned)grid_for((long long)N * H * W * C / 8), 256, 0, (cudaStream_t)stream,
                                   (const uint4 *)x, (uint4 *)y, N, H, W, C / 8));
@@ -883,7 +891,10 @@ int plbm_nn_assemble_host(const int8_t *mask, const float *features, void *y, in
 int plbm_nn_unet_forward(const void *x, void *const *acts, const plbm_nn_layer *layers, int levels, int N, int H, int W,
                          void *stream)
 {
-    if (!x || !acts || !layers || levels < 1) return PLBM_ERR_ARGUMENT;
+    if (!x || !acts || !layers || levels < 1 || levels > 31 || N < 1 || H < 1 || W < 1) return PLBM_ERR_ARGUMENT;
+    // every level's extents are halved exactly: up-sampling an odd one would read beyond its input
+    const unsigned odd = (1u << (levels - 1)) - 1;
+    if (((unsigned)H & odd) || ((unsigned)W & odd)) return PLBM_ERR_ARGUMENT;
     const plbm_nn_layer *layer = layers;
     void *const *next = acts;
     int rc = PLBM_OK;
@@ -896,7 +907,6 @@ int plbm_nn_unet_forward(const void *x, void *const *acts, const plbm_nn_layer *
     };
     const void *skip[32] = {};
     int width[32] = {};
-    if (levels > 32) return PLBM_ERR_ARGUMENT;
     const void *cur = x;
     for (int l = 0; l < levels; ++l) {
         const int h = H >> l, w = W >> l;

@@ -258,6 +258,7 @@ class NeuralOperator:
 
     def forward(self, x, n, h, w):
         """x: [n,h,w,4] bf16 input; returns the [n,h,w,3] prediction and keeps activations for backward.
+        h and w are multiples of 16 (four halvings); other extents raise RuntimeError.
 
         One native call launches every kernel (39 launches from Python took longer than they ran); the
         activations are pieces of one buffer, the prediction a tensor of its own."""
