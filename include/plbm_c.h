@@ -340,7 +340,7 @@ int plbm_nn_up2(const void *x, void *y, int N, int H, int W, int C, void *stream
 int plbm_nn_up2_bwd(const void *gy, void *gx, int N, int H, int W, int C, void *stream);
 int plbm_nn_add(const void *a, const void *b, void *y, long long n, void *stream);
 /* plbm_nn_assemble for four channels with the scalars on the host (3 N floats, read during the call):
- * no copy and no synchronisation.  y 8-byte aligned. */
+ * no copy and no synchronisation.  PLBM_ERR_ARGUMENT for extents below 1 or a y off an 8-byte boundary. */
 int plbm_nn_assemble_host(const int8_t *mask, const float *features, void *y, int N, int H, int W, void *stream);
 /* The operator's whole forward pass in one call: per level two convolutions and, but for the last, a
  * 2x2 average pooling; back up per level nearest upsampling, a convolution, the skip addition of the

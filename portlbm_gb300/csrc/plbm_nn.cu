@@ -865,7 +865,8 @@ int plbm_nn_add(const void *a, const void *b, void *y, long long n, void *stream
 
 int plbm_nn_assemble_host(const int8_t *mask, const float *features, void *y, int N, int H, int W, void *stream)
 {
-    if (!mask || !features || !y || N < 0 || H < 1 || W < 1 || (long long)H * W > 0x7fffffffll) return PLBM_ERR_ARGUMENT;
+    if (!mask || !features || !y || N < 1 || H < 1 || W < 1 || (long long)H * W > 0x7fffffffll) return PLBM_ERR_ARGUMENT;
+    if ((uintptr_t)y & 7u) return PLBM_ERR_ARGUMENT;   // a pixel is stored as one 8-byte unit
     const size_t pixels = (size_t)H * W;
     for (int n0 = 0; n0 < N; n0 += ASSEMBLE_SAMPLES) {
         const int n = N - n0 < ASSEMBLE_SAMPLES ? N - n0 : ASSEMBLE_SAMPLES;
