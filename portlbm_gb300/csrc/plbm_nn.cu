@@ -628,11 +628,17 @@ int bias_grad_v(const void *src, const void *skip, const void *y, void *out, flo
                               (const uint4 *)skip, (const uint4 *)y, (uint4 *)out, gb, (unsigned)P, H, W, CU));
 }
 
+// k_bias_grad_v applies: a block of 256 threads has at least one pixel lane.
+bool bias_vec(int C, long long elems, const void *a, const void *b = nullptr, const void *c = nullptr)
+{
+    return C <= 2048 && vec8(C, elems, a, b, c);
+}
+
 // gb[c] += sum over the P pixels of g[p][c]; with y, the ReLU backward of g first, in place (the
-// 16-byte kernel needs C a multiple of 8 and aligned buffers; y without them is applied by the caller).
+// 16-byte kernel needs what bias_vec says; y without that is applied by the caller).
 int bias_grad(const void *y, void *g, float *gb, long long P, int C, cudaStream_t s)
 {
-    if (vec8(C, P * C, g, y))
+    if (bias_vec(C, P * C, g, y))
         return y ? bias_grad_v<PLBM_NN_GRAD, true>(g, nullptr, y, g, gb, P, 1, 1, C, s)
                  : bias_grad_v<PLBM_NN_GRAD, false>(g, nullptr, nullptr, nullptr, gb, P, 1, 1, C, s);
     if (C <= 64 && vec8(8, P * C, g)) {   // a block's 2048 values hold each channel at least 32 times
@@ -761,7 +767,7 @@ int plbm_nn_conv_wgrad(const void *x, const void *g, float *gw, float *gb, int N
 int plbm_nn_relu_bwd_bias(const void *y, void *g, float *gb, long long P, int C, void *stream)
 {
     if (P <= 0 || C <= 0 || !gb) return PLBM_ERR_ARGUMENT;
-    if (!vec8(C, P * C, y, g)) {
+    if (!bias_vec(C, P * C, y, g)) {
         const int rc = plbm_nn_relu_bwd(y, g, P * C, stream);
         return rc == PLBM_OK ? bias_grad(nullptr, g, gb, P, C, (cudaStream_t)stream) : rc;
     }
@@ -776,8 +782,8 @@ int plbm_nn_relu_bwd_bias_from(int from, const void *g, const void *skip, const 
     if (P <= 0 || C <= 0 || !g || !y || !out || !gb || (pool && !skip)) return PLBM_ERR_ARGUMENT;
     if (!pool && !up && from != PLBM_NN_GRAD) return PLBM_ERR_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
-    // the 16-byte kernels; a block has at least one pixel lane, and every pixel a pooled one
-    if (C <= 2048 && vec8(C, P * C * (up ? 4 : 1), g, y, out) && vec8(C, P * C, skip) && !(pool && (H % 2 || W % 2))) {
+    // the 16-byte kernels; every pixel has a pooled one
+    if (bias_vec(C, P * C * (up ? 4 : 1), g, y, out) && vec8(C, P * C, skip) && !(pool && (H % 2 || W % 2))) {
         if (pool) return bias_grad_v<PLBM_NN_GRAD_POOL2, true>(g, skip, y, out, gb, P, H, W, C, s);
         if (up) return bias_grad_v<PLBM_NN_GRAD_UP2, true>(g, nullptr, y, out, gb, P, H, W, C, s);
         return bias_grad_v<PLBM_NN_GRAD, true>(g, nullptr, y, out, gb, P, 1, 1, C, s);
