@@ -15,16 +15,7 @@ template <int PREC, int L>
 static cudaError_t launch(const StepParams &p, int rows, cudaStream_t s)
 {
     const dim3 grid(two_step_blocks(p.W), (unsigned)((p.H + rows - 1) / rows));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(32, PAIR_WARPS);
-    cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_two_steps<PREC, L>, p, rows);
+    return launch_dependent(k_two_steps<PREC, L>, grid, dim3(32, PAIR_WARPS), 0, s, p, rows);
 }
 
 #define PLBM_PAIR_CASE(PR, LA) case (PR) * 3 + (LA): return launch<PR, LA>(p, rows, s);

@@ -9,6 +9,7 @@
 // There is no counterpart in the reference, which runs one domain per handler.
 #include "../../include/plbm_c.h"
 #include "plbm_consts.h"
+#include "plbm_dependent.cuh"
 #include "plbm_kernels.cuh"
 #include "plbm_launch.h"
 #include "plbm_pair.cuh"
@@ -467,21 +468,15 @@ struct plbm_batch {
     cudaError_t launch_two_steps(unsigned parity)
     {
         const plbm::BatchPairArgs a{ dom_d, pair_domain_d, pair_first_d, pair_rows, parity };
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(pair_blocks);
-        cfg.blockDim = dim3(32, plbm::PAIR_WARPS);
-        cfg.stream = stream;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
+        auto go = [&](void (*kernel)(plbm::BatchPairArgs)) {
+            return plbm::launch_dependent(kernel, dim3(pair_blocks), dim3(32, plbm::PAIR_WARPS), 0, stream, a);
+        };
         switch (prec) {
-        case PLBM_F32: return cudaLaunchKernelEx(&cfg, plbm::k_batch_two_steps<plbm::F32>, a);
-        case PLBM_F16S: return cudaLaunchKernelEx(&cfg, plbm::k_batch_two_steps<plbm::F16S>, a);
-        case PLBM_BF16S: return cudaLaunchKernelEx(&cfg, plbm::k_batch_two_steps<plbm::BF16S>, a);
-        case PLBM_F16C: return cudaLaunchKernelEx(&cfg, plbm::k_batch_two_steps<plbm::F16C>, a);
-        default: return cudaLaunchKernelEx(&cfg, plbm::k_batch_two_steps<plbm::F64_Q60>, a);
+        case PLBM_F32: return go(plbm::k_batch_two_steps<plbm::F32>);
+        case PLBM_F16S: return go(plbm::k_batch_two_steps<plbm::F16S>);
+        case PLBM_BF16S: return go(plbm::k_batch_two_steps<plbm::BF16S>);
+        case PLBM_F16C: return go(plbm::k_batch_two_steps<plbm::F16C>);
+        default: return go(plbm::k_batch_two_steps<plbm::F64_Q60>);
         }
     }
 

@@ -1,21 +1,13 @@
 // plbm_dispatch.cuh — maps runtime (precision, layout) to a template instantiation.
 #pragma once
+#include "plbm_dependent.cuh"
 #include "plbm_kernels.cuh"
 
 namespace plbm {
 // Launches a step kernel (one that calls step_begin) with programmatic stream serialization.
 inline cudaError_t launch_step_kernel(void (*kernel)(StepParams), dim3 grid, dim3 block, cudaStream_t s, const StepParams &p)
 {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, p);
+    return launch_dependent(kernel, grid, block, 0, s, p);
 }
 }  // namespace plbm
 

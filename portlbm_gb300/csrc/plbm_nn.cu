@@ -878,18 +878,10 @@ int plbm_nn_assemble_host(const int8_t *mask, const float *features, void *y, in
         const int n = N - n0 < ASSEMBLE_SAMPLES ? N - n0 : ASSEMBLE_SAMPLES;
         AssembleValues a{};
         for (int i = 0; i < 3 * n; ++i) a.v[i / 3][i % 3] = features[3 * n0 + i];
-        cudaLaunchConfig_t cfg{};
         const unsigned blocks = (unsigned)((pixels + 255) / 256);
-        cfg.gridDim = dim3(blocks < 256 ? blocks : 256, (unsigned)n);
-        cfg.blockDim = dim3(256);
-        cfg.stream = (cudaStream_t)stream;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_assemble_values, mask + n0 * pixels, a,
-                                                 (uint2 *)((__nv_bfloat16 *)y + 4 * n0 * pixels), n, (unsigned)pixels);
+        const cudaError_t e = nn_launch(k_assemble_values, dim3(blocks < 256 ? blocks : 256, (unsigned)n), 256, 0,
+                                        (cudaStream_t)stream, mask + n0 * pixels, a,
+                                        (uint2 *)((__nv_bfloat16 *)y + 4 * n0 * pixels), n, (unsigned)pixels);
         if (e != cudaSuccess) return PLBM_ERR_CUDA;
     }
     return PLBM_OK;

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "plbm_dependent.cuh"
+
 // The kernel's launch latency and set-up (barriers, tensor memory, descriptors) overlap the end of the
 // kernel before it in the stream: everything that reads or writes activations or parameters comes
 // after nn_begin, which waits for that kernel and lets the next one in.  Tensor memory is allocated
@@ -16,15 +18,5 @@ __device__ __forceinline__ void nn_begin()
 template <typename... P, typename... A>
 inline cudaError_t nn_launch(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A... args)
 {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    return plbm::launch_dependent(kernel, grid, dim3(block), smem, s, args...);
 }
