@@ -56,7 +56,9 @@ def build(force: bool = False, verbose: bool = False, checked: bool = False) -> 
     os.makedirs(build_dir, exist_ok=True)
     cc = nvcc()
     defs = ["-DPLBM_CHECKED"] if checked else []
-    common = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-lineinfo", *defs, "-I", CSRC,
+    # host arithmetic rounds every operation: gcc would fuse multiply-adds where the machine has them (aarch64),
+    # and the boundary constants would then differ in the last bit from one machine to the other
+    common = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off", "-lineinfo", *defs, "-I", CSRC,
               "-I", os.path.join(os.path.dirname(PKG), "include")]
     jobs = []
     for src in CU_SOURCES:
@@ -65,7 +67,7 @@ def build(force: bool = False, verbose: bool = False, checked: bool = False) -> 
     cuda_inc = os.path.join(os.path.dirname(os.path.dirname(cc)), "include")
     for src in CPP_SOURCES:
         obj = os.path.join(build_dir, src + ".o")
-        jobs.append(["g++", "-O2", "-std=c++17", "-fPIC", "-Wall", "-Wno-unknown-pragmas", *defs, "-I", cuda_inc,
+        jobs.append(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-Wall", "-Wno-unknown-pragmas", *defs, "-I", cuda_inc,
                      "-I", CSRC, "-c", os.path.join(CSRC, src), "-o", obj])
 
     def run(cmd):
