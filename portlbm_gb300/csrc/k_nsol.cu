@@ -16,6 +16,7 @@ cudaError_t launch_nsol(int prec, int lay, const StepParams &p, unsigned t, dim3
             case 5: return launch_step_kernel(k_nsol_even_staged<5>, grid, block, s, p);
             case 6: return launch_step_kernel(k_nsol_even_staged<6>, grid, block, s, p);
             case 7: return launch_step_kernel(k_nsol_even_staged<7>, grid, block, s, p);
+            case 8: return launch_step_kernel(k_nsol_even_staged<8>, grid, block, s, p);
             default: return cudaErrorInvalidValue;
             }
         }

@@ -56,6 +56,22 @@ inline void fill_q60_constants(StepParams &b)
     }
 }
 
+// Whether F64_STRICT steps try the integer-pipe collision (else F64_PLAIN: same values).  It takes nodes of
+// densities from about 0.4 to 1.8 and |jx| + |jy| below 0.2; a node outside pays for both collisions, 122
+// FP64 instructions instead of 97, so a channel of such nodes is better off without it (2000 x 500 at density
+// 2.5: 245 us a step, 197 without).  A channel starts from rest at density 1 and goes to its boundaries'
+// densities, at speeds that their ratio and the inlet's velocity set.  us a step after 8000 steps, 900 x 300
+// and 2000 x 500, plain 61.6 and 199.7: densities 1.4 / 1.0 21.6 and 67.7, 1.5 / 1.0 23.9 and 172, 1.6 / 1.0
+// 58.7 and 217, 1.4 / 1.35 20.8 and 66.5, 1.5 / 1.45 (the jump from rest is too much) 74.8 and 246, 1.0 / 0.7
+// 44.4 and 165, 1.0 / 0.5 71.3 and 236, 0.5 / 0.45 25.1 and 180, 0.4 / 0.35 64.9 and 240; velocity 0.15 27.0
+// and 184, 0.2 67.6 and 229.
+inline bool strict_pays(double omega, double rho_in, double vx_in, double vy_in, double rho_out, double vx_out, double vy_out)
+{
+    const double low = std::fmin(rho_in, rho_out), high = std::fmax(rho_in, rho_out);
+    const double speed = std::fmax(std::fabs(vx_in) + std::fabs(vy_in), std::fabs(vx_out) + std::fabs(vy_out));
+    return omega > 0 && low >= 0.45 && low <= 1.4 && high <= 1.5 && high <= 1.5 * low && speed < 0.18;
+}
+
 // Float constants of the FP32-arithmetic forms, rounded once from the double constants
 // (b.W, b.weight, b.feq_in, b.feq_out, b.rho_out, b.omega must be set).  For the shifted forms
 // the reference density is rho0(x') = a - g x' (see StepParams): profile = true gives the straight

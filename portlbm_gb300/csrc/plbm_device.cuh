@@ -90,6 +90,7 @@ __device__ __forceinline__ int cyd(int d) { return d / 3 - 1; }
 
 template <int PREC> struct Store;
 template <> struct Store<F64_STRICT> { using T = double; using C = double; };
+template <> struct Store<F64_PLAIN> { using T = double; using C = double; };
 template <> struct Store<F64_FAST> { using T = double; using C = double; };
 template <> struct Store<F32_REF> { using T = float; using C = float; };
 template <> struct Store<F32> { using T = float; using C = float; };
@@ -175,8 +176,8 @@ __device__ __forceinline__ double nan_guard(double v)
 // exact IEEE operation order, every operation rounded separately (no contraction).  Terms the
 // reference multiplies by a velocity component of 0 or +-1 are exact and are written as the
 // sums and negations they reduce to; the results are the same values.  This is the form for
-// populations outside the range of strict::fast_collide; it is bound by the FP64 pipe (97
-// instructions a node at about two lanes per cycle and SM).
+// populations outside the range of strict::fast_collide, and of the F64_PLAIN kernels; it is bound by
+// the FP64 pipe (97 instructions a node at about two lanes per cycle and SM).
 __device__ __forceinline__ Moments collide_f64_strict(double f[9], double omega)
 {
     double rho = f[0];
@@ -500,6 +501,7 @@ template <int PREC, bool FORMED = false>
 __device__ __forceinline__ MomentsOf<PREC> collide(typename Store<PREC>::C f[9], const StepParams &p)
 {
     if constexpr (PREC == F64_STRICT) return collide_strict(f, p.omega);
+    else if constexpr (PREC == F64_PLAIN) return collide_f64_strict(f, p.omega);
     else if constexpr (PREC == F64_FAST) return collide_f64_fast(f, p.omega);
     else if constexpr (PREC == F32_REF) return collide_f32_ref(f, p.omegaf);
     else if constexpr (PREC == F64_Q60) return collide_q60(f, p);
@@ -530,7 +532,7 @@ __device__ __forceinline__ void outlet_fill_float(float f[9], float hy, const St
 template <int PREC, bool BATCH = false>
 __device__ __forceinline__ void outlet_fill(typename Store<PREC>::C f[9], double jyo, const StepParams &p)
 {
-    if constexpr (PREC == F64_STRICT) {
+    if constexpr (PREC == F64_STRICT || PREC == F64_PLAIN) {
         const double xv = __dadd_rn(-p.rho_out,
                                     __dadd_rn(__dadd_rn(__dadd_rn(f[1], f[4]), f[7]),
                                               __dmul_rn(2.0, __dadd_rn(__dadd_rn(f[8], f[5]), f[2]))));

@@ -13,7 +13,7 @@ inline cudaError_t launch_step_kernel(void (*kernel)(StepParams), dim3 grid, dim
 
 #define PLBM_CASE(KER, PR, LA) case (PR) * 3 + (LA): return launch_step_kernel(KER<PR, LA>, grid, block, s, p);
 #define PLBM_ALL_CASES(KER) PLBM_ALL_CASES_2(KER, KER)
-// BOUND: the kernel of the F64_STRICT and F64_Q60 forms
+// BOUND: the kernel of the F64_STRICT, F64_PLAIN and F64_Q60 forms
 #define PLBM_ALL_CASES_2(BOUND, KER)                                                          \
     PLBM_CASE(BOUND, 0, 0) PLBM_CASE(BOUND, 0, 1) PLBM_CASE(BOUND, 0, 2)                       \
     PLBM_CASE(KER, 1, 0) PLBM_CASE(KER, 1, 1) PLBM_CASE(KER, 1, 2)                             \
@@ -22,7 +22,8 @@ inline cudaError_t launch_step_kernel(void (*kernel)(StepParams), dim3 grid, dim
     PLBM_CASE(KER, 4, 0) PLBM_CASE(KER, 4, 1) PLBM_CASE(KER, 4, 2)                             \
     PLBM_CASE(KER, 5, 0) PLBM_CASE(KER, 5, 1) PLBM_CASE(KER, 5, 2)                             \
     PLBM_CASE(BOUND, 6, 0) PLBM_CASE(BOUND, 6, 1) PLBM_CASE(BOUND, 6, 2)                       \
-    PLBM_CASE(KER, 7, 0) PLBM_CASE(KER, 7, 1) PLBM_CASE(KER, 7, 2)
+    PLBM_CASE(KER, 7, 0) PLBM_CASE(KER, 7, 1) PLBM_CASE(KER, 7, 2)                             \
+    PLBM_CASE(BOUND, 8, 0) PLBM_CASE(BOUND, 8, 1) PLBM_CASE(BOUND, 8, 2)
 
 // The porous gather of the shifted forms (f32, f16s, bf16s, f16c; the unshifted forms have one gather).
 #define PLBM_POROUS_CASE(KER, PR, LA) case (PR) * 3 + (LA): return launch_step_kernel(KER<PR, LA, true>, grid, block, s, p);

@@ -453,6 +453,7 @@ struct plbm_handler {
     int alg = 0, lay = 0, prec = 0;
     int W = 0, H = 0, P = 0;
     unsigned long long N = 0;
+    int step_prec = PLBM_F64_STRICT;   // form of the step kernels: prec, or F64_PLAIN for F64_STRICT
     int outlet_mode = 0;
     // debugMode on nptl / lptl: the reference's unfused stream / observables / collide kernels
     bool debug = false;
@@ -864,10 +865,10 @@ struct plbm_handler {
         if (alg == 2) { p.halo_in = (double *)halo[par]; p.halo_out = (double *)halo[par ^ 1u]; }
         if (debug) return plbm::launch_debug_step(prec, lay, alg == 1, p, block, stream);
         switch (alg) {
-        case 0: return plbm::launch_nptl(prec, lay, p, grid, block, stream, porous, vec_rows);
-        case 1: return plbm::launch_lptl(prec, lay, p, grid, block, stream, porous);
-        case 2: return plbm::launch_npol(prec, lay, p, grid, block, stream);
-        default: return plbm::launch_nsol(prec, lay, p, t, grid, block, stream);
+        case 0: return plbm::launch_nptl(step_prec, lay, p, grid, block, stream, porous, vec_rows);
+        case 1: return plbm::launch_lptl(step_prec, lay, p, grid, block, stream, porous);
+        case 2: return plbm::launch_npol(step_prec, lay, p, grid, block, stream);
+        default: return plbm::launch_nsol(step_prec, lay, p, t, grid, block, stream);
         }
     }
 
@@ -893,8 +894,11 @@ struct plbm_handler {
     //  * nptl's 2-byte forms step vectorised rows in the stream layout from four fifths of L2 on; on
     //    smaller domains, where the few warps of 256 nodes wait, the scalar kernel (1000 x 300 f16s 9.3
     //    against 6.0 us, 2000 x 500 14.3 / 11.3, 3000 x 1000 32.8 / 34.1).
+    //  * F64_STRICT: whether the integer-pipe collision is tried (strict_pays).
     void choose_kernels()
     {
+        step_prec = prec != PLBM_F64_STRICT || plbm::strict_pays(base.omega, props.irho, props.ivx, props.ivy, props.orho,
+                                                                 props.ovx, props.ovy) ? prec : (int)plbm::F64_PLAIN;
         int l2 = 0;
         cuda_check(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, opt.device), "device attribute");
         const unsigned long long lattices = 2 * 9ull * N * storage_bytes(prec), cache = (unsigned long long)l2;

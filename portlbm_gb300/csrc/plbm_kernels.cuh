@@ -776,8 +776,9 @@ __device__ __forceinline__ void nsol_even_collision_staged(const StepParams &p)
 // The staged even step as its own kernel (launched by launch_nsol for 32 x NSOL_STAGE_ROWS blocks
 // in the collision layout): 256 threads, four resident blocks (the 64-register cap an unbounded
 // kernel gets), five for the Q60 form (48 registers, measured faster), three for F64_STRICT.  The
-// other nsol kernels keep no launch bounds, except those of F64_STRICT and F64_Q60 (NsolBlocks): a bound above 256 threads let the compiler take 98 registers for the stream
-// layout's even step and halved its resident blocks.
+// other nsol kernels keep no launch bounds, except those of F64_STRICT, F64_PLAIN and F64_Q60 (NsolBlocks): a
+// bound above 256 threads let the compiler take 98 registers for the stream layout's even step and halved
+// its resident blocks.
 template <int PREC>
 __global__ void __launch_bounds__(256, PREC == F64_Q60 ? 5 : PREC == F64_STRICT ? 3 : 4) k_nsol_even_staged(StepParams p)
 {
@@ -842,7 +843,7 @@ __device__ __forceinline__ void nsol_odd_gather(CT<PREC> f[9], unsigned long lon
 }
 
 // Q60: five blocks (48 registers): 8192 x 8192 stream 44.2 k MLUPS, 41.0 k without a bound; three, four
-// and six blocks measured 15, 6 and 2 % slower.
+// and six blocks measured 15, 6 and 2 % slower.  F64_PLAIN: 2000 x 500 stream 192 us a step, 202 without one.
 template <int PREC> struct NsolBlocks { static constexpr int value = PREC == F64_Q60 ? 5 : 3; };
 template <int PREC, int L> __global__ void k_nsol_even(StepParams p) { nsol_even_step<PREC, L>(p); }
 template <int PREC, int L> __global__ void __launch_bounds__(256, NsolBlocks<PREC>::value) k_nsol_even_bound(StepParams p)

@@ -8,6 +8,7 @@
 // needs — the outlet's jy column of the previous step, two parities — lives in the fixed device
 // array below.
 #include "../../include/plbm_c.h"
+#include "plbm_consts.h"
 #include "plbm_kernels.cuh"
 #include "plbm_launch.h"
 
@@ -34,6 +35,7 @@ thread_local char g_err[256];
 // Solid-source bits are derived from the caller's flag grid on the fly (no link array).  One rule
 // for both uses of a flag: 0 is fluid, any other value solid (a node that does not update is also
 // a bounce-back source for its neighbours).
+template <int PREC>   // F64_STRICT or F64_PLAIN
 __global__ void k_nptl_noalloc(plbm::StepParams p, const int8_t *flags)
 {
     using namespace plbm;
@@ -51,12 +53,12 @@ __global__ void k_nptl_noalloc(plbm::StepParams p, const int8_t *flags)
     const unsigned long long n = (unsigned long long)xi + (unsigned long long)yi * p.P;
     double f[9];
 #pragma unroll
-    for (int d = 0; d < 9; ++d) f[d] = pull_one<F64_STRICT, STREAM>(p.lat0, n, xi, yi, d, lk, p);
-    if (is_outlet_row(xi, yi, p)) outlet_fill<F64_STRICT>(f, jy_prev_at(p, yi), p);
-    const MomentsS m = collide<F64_STRICT>(f, p);
+    for (int d = 0; d < 9; ++d) f[d] = pull_one<PREC, STREAM>(p.lat0, n, xi, yi, d, lk, p);
+    if (is_outlet_row(xi, yi, p)) outlet_fill<PREC>(f, jy_prev_at(p, yi), p);
+    const MomentsOf<PREC> m = collide<PREC>(f, p);
 #pragma unroll
-    for (int d = 0; d < 9; ++d) st<F64_STRICT>(p.lat1, lidx<STREAM>(n, d, p.N), d, f[d], p);
-    observables<F64_STRICT>(m, xi, yi, p);
+    for (int d = 0; d < 9; ++d) st<PREC>(p.lat1, lidx<STREAM>(n, d, p.N), d, f[d], p);
+    observables<PREC>(m, xi, yi, p);
 }
 
 __global__ void k_noalloc_clear(double *scratch, unsigned n)
@@ -115,7 +117,11 @@ extern "C" int plbm_nptl_steps_noalloc(const plbm_noalloc_args *a)
         std::lock_guard<std::mutex> g(g_mu);
         if (!g_scratch_addr[dev]) {
             void *ptr = nullptr;
-            const cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
+            cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
+            // both forms of the kernel are loaded now, so that a later call with other boundaries loads nothing
+            cudaFuncAttributes attr;
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, k_nptl_noalloc<plbm::F64_STRICT>);
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, k_nptl_noalloc<plbm::F64_PLAIN>);
             if (e != cudaSuccess) return fail(PLBM_ERR_CUDA, cudaGetErrorString(e));
             g_scratch_addr[dev] = static_cast<double *>(ptr);
         }
@@ -149,6 +155,8 @@ extern "C" int plbm_nptl_steps_noalloc(const plbm_noalloc_args *a)
         }
     }
     const dim3 block(32, 8), grid((W + 31) / 32, (H + 7) / 8);
+    const bool fast = plbm::strict_pays(p.omega, a->inlet_density, a->inlet_velocity_x, a->inlet_velocity_y,
+                                        a->outlet_density, a->outlet_velocity_x, a->outlet_velocity_y);
     void *lat[2] = { a->lattice0, a->lattice1 };
     for (unsigned k = 0; k < a->steps && e == cudaSuccess; ++k) {
         const unsigned t = a->first_step + k, par = t & 1u;
@@ -157,7 +165,8 @@ extern "C" int plbm_nptl_steps_noalloc(const plbm_noalloc_args *a)
         p.jy_prev = scratch + (size_t)par * H;
         p.jy_next = scratch + (size_t)(par ^ 1u) * H;
         p.write_results = (k + 1 == a->steps);
-        k_nptl_noalloc<<<grid, block, 0, s>>>(p, a->flags);
+        if (fast) k_nptl_noalloc<plbm::F64_STRICT><<<grid, block, 0, s>>>(p, a->flags);
+        else k_nptl_noalloc<plbm::F64_PLAIN><<<grid, block, 0, s>>>(p, a->flags);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return fail(PLBM_ERR_CUDA, cudaGetErrorString(e));

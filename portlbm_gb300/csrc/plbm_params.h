@@ -6,7 +6,8 @@
 namespace plbm {
 
 enum Layout { COLLISION = 0, STREAM = 1, BUNDLE = 2 };
-enum Precision { F64_STRICT = 0, F64_FAST = 1, F32_REF = 2, F32 = 3, F16S = 4, BF16S = 5, F64_Q60 = 6, F16C = 7 };
+enum Precision { F64_STRICT = 0, F64_FAST = 1, F32_REF = 2, F32 = 3, F16S = 4, BF16S = 5, F64_Q60 = 6, F16C = 7,
+                 F64_PLAIN = 8 };   // F64_STRICT's steps with the collision on the FP64 pipe alone (strict_pays)
 
 constexpr uint16_t LINK_FLUID = 1u << 4;
 // Set by k_links on the nodes of the first and last inner row and column: with it, an interior
