@@ -805,10 +805,22 @@ struct plbm_handler {
         // Small domains: blocks are halved, down to 64 threads, until there are four for every SM, so
         // that all SMs share the work evenly (400 x 100: f64_strict 6.5 -> 6.0 us a step, f64_q60
         // 3.6 -> 3.2; 62 x 30: 5.5 -> 4.7 and 2.9 -> 2.6).  npol's blocks are its tiles and stay.
+        // Records (the collision layout) of the shifted forms and of F64_Q60 keep blocks of 128: a block's or a
+        // warp's records are written together, and blocks of 64 cost more than they share out.  The other forms'
+        // steps are bound by the FP64 pipe and better shared out (f64_strict 400 x 100: nsol 7.2 us a step with
+        // 64, 8.1 with 128), but for lptl's F64_STRICT.  us a step with 64 / 128: f64_q60 nptl 1001 x 67 4.55 /
+        // 3.85 (62 x 30, on few SMs, 2.93 / 3.12), lptl 500 x 150 5.57 / 4.76, nsol 803 x 60 4.80 / 4.24; bf16s
+        // nsol 1200 x 60 5.5 / 5.0; f64_strict lptl 500 x 150 9.0 / 7.9.  Two cases are better with still larger
+        // blocks: lptl f32 with 256 (512 x 256: 6.0, 5.1 with 256), nsol f64_q60 with three blocks for two SMs
+        // (1200 x 60 porous: 6.28, 5.54 with 256).
         if (alg != 2) {
+            const bool records = lay == plbm::COLLISION, q60 = records && prec == PLBM_F64_Q60;
+            const bool wide = records && (shifted || q60 || (alg == 1 && prec == PLBM_F64_STRICT));
+            unsigned least = !wide ? 64 : alg == 1 && prec == PLBM_F32 ? 256 : 128;
             int sms = 0;
             cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opt.device), "device attribute");
-            while ((unsigned long long)grid.x * grid.y < 4ull * sms && block.x * block.y > 64) {
+            const unsigned long long wanted = q60 && alg == 3 ? 3ull * sms / 2 : 4ull * sms;
+            while ((unsigned long long)grid.x * grid.y < wanted && block.x * block.y > least) {
                 if (alg == 1) {
                     block.x = std::max(64u, block.x / 64 * 32);
                     grid.x = (unsigned)((N + (unsigned long long)block.x * ny - 1) / ((unsigned long long)block.x * ny));
@@ -817,6 +829,7 @@ struct plbm_handler {
                     else block.x = block.x / 64 * 32;
                     grid = dim3((W + block.x - 1) / block.x, (H + block.y * ny - 1) / (block.y * ny));
                 }
+                if (q60 && alg == 0 && 2ull * grid.x * grid.y < (unsigned)sms) least = 64;
             }
         }
         if (alg == 2) {
