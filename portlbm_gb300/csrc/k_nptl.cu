@@ -6,6 +6,7 @@ namespace plbm {
 cudaError_t launch_nptl(int prec, int lay, const StepParams &p, dim3 grid, dim3 block, cudaStream_t s, bool porous,
                         bool vec_rows)
 {
+    static_assert(VEC_ROW_NODES == 32 * VEC, "a warp's nodes");
     const bool two_byte = vec_rows && (prec == F16S || prec == BF16S || prec == F16C);
     const dim3 vb(32, VEC_ROWS), vg((unsigned)((p.P + 32 * VEC - 1) / (32 * VEC)), (unsigned)((p.H + VEC_ROWS - 1) / VEC_ROWS));
     // 2-byte storage in the stream layout on porous geometries: vectorised rows with the bounce-back

@@ -458,7 +458,8 @@ struct plbm_handler {
     // debugMode on nptl / lptl: the reference's unfused stream / observables / collide kernels
     bool debug = false;
     int pair_rows = 0;     // rows a warp of the two-step kernel marches over; 0: one step a launch
-    bool vec_rows = false; // nptl, 2-byte storage, stream layout: vectorised rows
+    bool vec_rows = false, vec_results = false;   // nptl, 2-byte storage, stream layout: plain steps and steps
+                                                  // with results by vectorised rows
     bool porous = false;   // nptl/lptl shifted forms: the obstacle-select gather (PLBM_GATHER_POROUS)
 
     cudaStream_t stream = nullptr;
@@ -878,7 +879,7 @@ struct plbm_handler {
         if (alg == 2) { p.halo_in = (double *)halo[par]; p.halo_out = (double *)halo[par ^ 1u]; }
         if (debug) return plbm::launch_debug_step(prec, lay, alg == 1, p, block, stream);
         switch (alg) {
-        case 0: return plbm::launch_nptl(step_prec, lay, p, grid, block, stream, porous, vec_rows);
+        case 0: return plbm::launch_nptl(step_prec, lay, p, grid, block, stream, porous, results ? vec_results : vec_rows);
         case 1: return plbm::launch_lptl(step_prec, lay, p, grid, block, stream, porous);
         case 2: return plbm::launch_npol(step_prec, lay, p, grid, block, stream);
         default: return plbm::launch_nsol(step_prec, lay, p, t, grid, block, stream);
@@ -906,7 +907,12 @@ struct plbm_handler {
     //    strips, 64 x 3000, 8.1 / 8.4).
     //  * nptl's 2-byte forms step vectorised rows in the stream layout from four fifths of L2 on; on
     //    smaller domains, where the few warps of 256 nodes wait, the scalar kernel (1000 x 300 f16s 9.3
-    //    against 6.0 us, 2000 x 500 14.3 / 11.3, 3000 x 1000 32.8 / 34.1).
+    //    against 6.0 us, 2000 x 500 14.3 / 11.3, 3000 x 1000 32.8 / 34.1).  Porous ones, whose solid nodes
+    //    cost the scalar kernel more, from a quarter of L2 on where the rows fill the warps (f16s 1200 x 800
+    //    12.8 / 13.2, 2000 x 500 12.1 / 13.4, 1700 x 1000 17.9 / 20.9, 1300 x 900 15.1 / 15.7, but 1000 x 800
+    //    11.6 / 11.4, and 300 x 4000, rows of 320 in 512, 22.6 / 19.6; f16c 2000 x 500 16.2 / 17.2, 1500 x 1000
+    //    22.9 / 24.3, but 1300 x 900 20.9 / 20.2, 1200 x 800 17.1 / 16.9); not for results (f16s 1600 x 1200 a
+    //    step with results 137 / 107).
     //  * F64_STRICT: whether the integer-pipe collision is tried (strict_pays).
     void choose_kernels()
     {
@@ -916,7 +922,9 @@ struct plbm_handler {
         cuda_check(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, opt.device), "device attribute");
         const unsigned long long lattices = 2 * 9ull * N * storage_bytes(prec), cache = (unsigned long long)l2;
         const bool shifted = prec == PLBM_F32 || prec == PLBM_F16S || prec == PLBM_BF16S || prec == PLBM_F16C;
-        vec_rows = lattices > cache / 5 * 4;
+        const int in_warps = (P + plbm::VEC_ROW_NODES - 1) / plbm::VEC_ROW_NODES * plbm::VEC_ROW_NODES;   // of a row
+        vec_results = vec_rows = lattices > cache / 5 * 4;
+        if (porous && lattices > cache / 4 && P * 20 > in_warps * (prec == PLBM_F16C ? 19 : 17)) vec_rows = true;
         pair_rows = 0;
         if (!two_lattice() || debug) return;
         int sms = 0;

@@ -9,7 +9,8 @@ namespace plbm {
 // One timestep of algorithm `alg` (0 nptl, 1 lptl, 2 npol, 3 nsol) for precision `prec` and
 // layout `lay`; `t` is the absolute step index (selects the nsol parity kernel).
 // porous: the obstacle-select gather of the shifted forms (f32, f16s, bf16s)
-// vec_rows: the vectorised rows of the 2-byte forms (stream layout)
+// vec_rows: the vectorised rows of the 2-byte forms (stream layout), VEC_ROW_NODES of a row to a warp
+constexpr int VEC_ROW_NODES = 256;
 cudaError_t launch_nptl(int prec, int lay, const StepParams &p, dim3 grid, dim3 block, cudaStream_t s, bool porous,
                         bool vec_rows);
 cudaError_t launch_lptl(int prec, int lay, const StepParams &p, dim3 grid, dim3 block, cudaStream_t s, bool porous);
