@@ -7,6 +7,7 @@ namespace plbm {
 
 unsigned two_step_blocks(int W)
 {
+    static_assert(TWO_STEP_COLUMNS == PAIR_COLUMNS, "a strip's columns");
     const int strips = (W + PAIR_COLUMNS - 1) / PAIR_COLUMNS;
     return (unsigned)((strips + PAIR_WARPS - 1) / PAIR_WARPS);
 }

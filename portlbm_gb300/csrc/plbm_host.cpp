@@ -886,11 +886,40 @@ struct plbm_handler {
         }
     }
 
+    // Whether a shifted form's lattices beyond half of L2 step two at a time: not where rows are so narrow that
+    // their strips are many more than a single step's warps, nor in the forms and layouts whose single steps are
+    // as good up to a larger size.  us a step singly / two at a time:
+    //  * nptl's records of open channels (f32 1200 x 800 11.9 / 15.1, 1300 x 900 14.4 / 17.6) from three
+    //    quarters of L2 on, but narrow ones, whose single steps are slow, at once (f32 250 x 4688 20.7 / 18.5;
+    //    f16c 80 x 22917 43.8 / 38.5); rows of exactly a warp in two strips are full (bf16s 32 x 64062 47.5 /
+    //    50.5, f16c 52.6 / 66.4);
+    //  * the other layouts: two strips for one warp (W = 31, 32: f32 37501 rows 27.9 / 31.0, bf16s 64062 rows
+    //    43.1 / 54.0, f16c 53.4 / 70.2) but for f16s (66.2 / 58.9) and porous bundles (f32 31.1 / 29.7); f16c of
+    //    open channels, whose conversions the extra strips repeat, from five strips for four warps on up to one
+    //    and a half times L2 (61 x 32031 43.0 / 51.7, 61 x 64062 88.8 / 101, 121 x 17188 40.1 / 45.0, but 95 x
+    //    62500 118 / 103).  nptl's vectorised rows of the 2-byte forms are slower than two steps a launch at any
+    //    width (f16s 61 x 34376 106 / 45).
+    bool two_steps_pay(int strips, int warps, unsigned long long lattices, unsigned long long cache) const
+    {
+        const bool narrow = 2 * strips > 3 * warps, wide_values = prec == PLBM_F32 || prec == PLBM_F16C;
+        if (lay == plbm::COLLISION) {
+            if (porous) return true;
+            if (W == 32) return prec == PLBM_F32 || prec == PLBM_F16S;
+            return alg != 0 || !wide_values || W <= 512 || lattices > cache / 4 * 3;
+        }
+        if (prec == PLBM_F16S || (alg == 0 && lay == plbm::STREAM && prec != PLBM_F32)) return true;
+        if (prec == PLBM_F16C && !porous && 5 * strips > 6 * warps && lattices < cache / 2 * 3) return false;
+        return !narrow || (lay == plbm::BUNDLE && porous && prec != PLBM_F16C);
+    }
+
     // The kernels of nptl and lptl that pay on domains whose two lattices outgrow L2, or that are small:
-    //  * plain steps two a launch.  Shifted forms from half of L2 on: f32 72 MB of lattices 10.7 us a step
+    //  * plain steps two a launch.  Shifted forms from half of L2 on (but see two_steps_pay): f32 72 MB of lattices 10.7 us a step
     //    singly against 10.5, 111 MB 19.4 / 14.6, 216 MB 38.1 / 27.0; f16s 72 MB 20.6 / 19.5, 108 MB
     //    36.3 / 27.3; below (1000 x 300) 4.6 / 5.4.  F64_Q60, bound by instructions as much as by HBM,
-    //    from eight times L2 on: 1.2 GB 180 / 173, 2.4 GB 433 / 373, but 144 MB 26.2 / 30.5.  The rows of
+    //    from eight times L2 on: 1.2 GB 180 / 173, 2.4 GB 433 / 373, but 144 MB 26.2 / 30.5; where strips are
+    //    many more than warps not (1.15 GB, nptl: 250 columns, 9 strips for 8 warps, 199 / 219, 155 columns, 6
+    //    for 5, 221 / 241, but 200 columns, 7 for 7, 211 / 205 and lptl records of 250 columns 232 / 223; 2.3 GB:
+    //    250 columns 422 / 423, porous 453 / 431).  The rows of
     //    a strip trade rows done twice against blocks enough for every SM: shifted 4 up to 4 M nodes
     //    (3 M: 27.0, with 8 rows 28.0), 8 up to 32 M (8 M: 59.9, with 4 rows 61.6), 16 above (67 M: 429,
     //    with 8 rows 445); Q60 16 up to 16 M, 32 above (67 M: 1222, with 16 rows 1254).
@@ -903,8 +932,9 @@ struct plbm_handler {
     //    And shifted records of porous domains at any size, two rows a strip: a single step's warps that hold
     //    a solid node, most of them, store their records value by value (512 x 256: f32 4.64 / 3.51, f16s
     //    5.25 / 3.89; 700 x 300: f32 6.05 / 4.01, f16s 6.84 / 4.56, f16c 6.67 / 5.71; 1000 x 800: 13.1 / 9.8,
-    //    14.7 / 10.5, 16.3 / 14.6; but in an open channel 1024 x 512 f32 7.44 / 8.54, and f16c with few
-    //    strips, 64 x 3000, 8.1 / 8.4).
+    //    14.7 / 10.5, 16.3 / 14.6; but in an open channel 1024 x 512 f32 7.44 / 8.54).  f16c only up to six
+    //    strips for five warps (lptl 100 x 1000, 4 for 4, 5.6 / 4.7, 250 x 400, 9 for 8, 5.0 / 4.8; 128 x 1500,
+    //    5 for 4, 6.3 / 7.2, 64 x 3000, 3 for 2, 6.7 / 8.4).
     //  * nptl's 2-byte forms step vectorised rows in the stream layout from four fifths of L2 on; on
     //    smaller domains, where the few warps of 256 nodes wait, the scalar kernel (1000 x 300 f16s 9.3
     //    against 6.0 us, 2000 x 500 14.3 / 11.3, 3000 x 1000 32.8 / 34.1).  Porous ones, whose solid nodes
@@ -930,9 +960,15 @@ struct plbm_handler {
         int sms = 0;
         cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opt.device), "device attribute");
         if (shifted && N <= (1ull << 16) && (unsigned long long)plbm::two_step_blocks(W) * H <= 8ull * sms) pair_rows = 1;
-        if (shifted && porous && lay == plbm::COLLISION && !pair_rows && (prec != PLBM_F16C || W >= 256)) pair_rows = 2;
-        if (shifted && lattices > cache / 2) pair_rows = N < (1ull << 22) ? 4 : N < (1ull << 25) ? 8 : 16;
-        if (prec == PLBM_F64_Q60 && lattices > 8 * cache) pair_rows = N < (1ull << 24) ? 16 : 32;
+        // warps a row takes in two-step launches (strips) and in single steps
+        const int strips = (W + plbm::TWO_STEP_COLUMNS - 1) / plbm::TWO_STEP_COLUMNS, warps = P / 32;
+        const bool records = lay == plbm::COLLISION;
+        if (shifted && porous && records && !pair_rows && (prec != PLBM_F16C || 5 * strips <= 6 * warps)) pair_rows = 2;
+        if (shifted && lattices > cache / 2 && two_steps_pay(strips, warps, lattices, cache))
+            pair_rows = N < (1ull << 22) ? 4 : N < (1ull << 25) ? 8 : 16;
+        if (prec == PLBM_F64_Q60 && lattices > 8 * cache &&
+            100 * strips <= (lattices > 16 * cache || (alg == 1 && records) ? 115 : 110) * warps)
+            pair_rows = N < (1ull << 24) ? 16 : 32;
         // the kernel's offsets (bytes, values of 8-byte storage) and its grid height are 32 and 16 bits
         const unsigned long long offsets = 9ull * N * (prec == PLBM_F64_Q60 ? 1 : storage_bytes(prec));
         if (pair_rows && (offsets >= (1ull << 32) || (H + pair_rows - 1) / pair_rows > 65535)) pair_rows = 0;

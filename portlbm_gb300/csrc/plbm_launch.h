@@ -18,6 +18,7 @@ cudaError_t launch_lptl(int prec, int lay, const StepParams &p, dim3 grid, dim3 
 // results).  rows: rows of the domain a warp marches over.
 cudaError_t launch_two_steps(int prec, int lay, const StepParams &p, int rows, cudaStream_t s);
 unsigned two_step_blocks(int W);   // of one row of strips
+constexpr int TWO_STEP_COLUMNS = 30;   // columns a strip, the work of a warp, writes
 // counts[0] = 32-node row segments holding fluid, counts[1] = those mixing interior nodes with and
 // without a solid neighbour
 cudaError_t launch_count_obstacle_nodes(const uint16_t *links, int W, int H, int P, unsigned long long *counts,
