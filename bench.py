@@ -225,11 +225,12 @@ def device_run(plbm, precision, alg, lay, w, h, mask, steps, warmup, tau=None, w
         props.relaxation_time = float(tau)
     hd = plbm.create_handler(props, precision=precision, mask=mask)
     hd.run_steps(warmup)
-    launches = hd.run_launches(steps)
+    launches = hd.launches()
     t0 = time.time()
     ms = hd.run_steps(steps)
     if window is not None:
         window[:] = [t0, time.time()]
+    launches = hd.launches() - launches
     return ms, launches, hd
 
 

@@ -195,6 +195,9 @@ int plbm_launches_per_step(plbm_handler *h, unsigned *n);
  * two a launch on large domains of the shifted forms and of the Q60 form, and on small domains and
  * porous records of the shifted forms. */
 int plbm_run_launches(plbm_handler *h, unsigned n, unsigned *launches);
+/* Kernels of steps that the handler has launched since it was created, counted as they are issued (a graph
+ * replay by the kernels it holds). */
+int plbm_launches(plbm_handler *h, unsigned long long *n);
 /* Algorithmic HBM bytes per node update of the hot kernel (9 loads + 9 stores). */
 int plbm_bytes_per_node(plbm_handler *h, double *bytes);
 /* Reads back the total fluid mass and momentum (FP64 reductions on the GPU). */
@@ -299,6 +302,8 @@ int plbm_batch_autotune(plbm_batch *b, unsigned steps, int *tile_w, int *tile_h,
 int plbm_batch_run(plbm_batch *b, unsigned steps, int mode, double *ms_per_step);
 int plbm_batch_results(plbm_batch *b, unsigned domain, int which, double *out);
 int plbm_batch_info(plbm_batch *b, unsigned long long *nodes, unsigned *tiles);
+/* Kernels of steps launched since the batch was created (as plbm_launches). */
+int plbm_batch_launches(plbm_batch *b, unsigned long long *n);
 const char *plbm_batch_last_error(void);
 
 /* ---- learned warm start (no counterpart in the reference) -----------------------------------

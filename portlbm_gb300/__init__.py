@@ -118,6 +118,7 @@ _SIGS = {
     "plbm_sync_results": (ctypes.c_int, [ctypes.c_void_p]),
     "plbm_gather_form": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)]),
     "plbm_run_launches": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint, ctypes.POINTER(ctypes.c_uint)]),
+    "plbm_launches": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_ulonglong)]),
     "plbm_launches_per_step": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint)]),
     "plbm_bytes_per_node": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_double)]),
     "plbm_mass_momentum": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_double)]),
@@ -461,6 +462,12 @@ class AlgorithmHandler:
         self._call("plbm_launches_per_step", ctypes.byref(v))
         return v.value
 
+    def launches(self) -> int:
+        """Kernels of steps launched so far, counted as they are issued."""
+        v = ctypes.c_ulonglong()
+        self._call("plbm_launches", ctypes.byref(v))
+        return v.value
+
     def run_launches(self, steps: int) -> int:
         """Kernel launches the next run_steps(steps) issues (plain steps may run two a launch)."""
         v = ctypes.c_uint()
@@ -495,6 +502,7 @@ class Batch:
                 ("plbm_batch_results", ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint, ctypes.c_int, ctypes.c_void_p]),
                 ("plbm_batch_info", ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_ulonglong),
                                                    ctypes.POINTER(ctypes.c_uint)]),
+                ("plbm_batch_launches", ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_ulonglong)]),
                 ("plbm_batch_last_error", ctypes.c_char_p, [])):
             fn = getattr(lib, name)
             fn.restype = res
@@ -547,6 +555,12 @@ class Batch:
         n, t = ctypes.c_ulonglong(), ctypes.c_uint()
         self._ok(self._lib.plbm_batch_info(self._h, ctypes.byref(n), ctypes.byref(t)))
         return n.value, t.value
+
+    def launches(self) -> int:
+        """Kernels of steps launched so far, counted as they are issued."""
+        n = ctypes.c_ulonglong()
+        self._ok(self._lib.plbm_batch_launches(self._h, ctypes.byref(n)))
+        return n.value
 
 
 def write_npy(path, array) -> None:

@@ -332,6 +332,7 @@ struct plbm_batch {
     cudaStream_t stream = nullptr;
     cudaGraphExec_t gexec = nullptr;
     unsigned graph_steps = 0;
+    unsigned long long issued = 0, graph_kernels = 0;   // kernels of steps; those of a replay of gexec
     int pair_rows = 0;             // rows of a two-step launch's pieces; 0: single steps only (offsets too wide)
     unsigned pair_blocks = 0;
     unsigned *pair_domain_d = nullptr, *pair_first_d = nullptr;
@@ -409,6 +410,7 @@ struct plbm_batch {
         if (e != cudaSuccess) return e;
         const plbm::BatchArgs a = args(step & 1u, write_results);
         const dim3 block(tile_w, tile_h);
+        ++issued;
         switch (prec) {
         case PLBM_F32: plbm::k_batch<plbm::F32><<<blocks, block, 0, stream>>>(a); break;
         case PLBM_F16S:
@@ -468,6 +470,7 @@ struct plbm_batch {
     cudaError_t launch_two_steps(unsigned parity)
     {
         const plbm::BatchPairArgs a{ dom_d, pair_domain_d, pair_first_d, pair_rows, parity };
+        ++issued;
         auto go = [&](void (*kernel)(plbm::BatchPairArgs)) {
             return plbm::launch_dependent(kernel, dim3(pair_blocks), dim3(32, plbm::PAIR_WARPS), 0, stream, a);
         };
@@ -497,6 +500,7 @@ struct plbm_batch {
     {
         const plbm::BatchArgs a = args(step & 1u, write_results);
         const dim3 block(32, 4);
+        issued += n_domains();
         for (unsigned i = 0; i < n_domains(); ++i) {
             const dim3 grid((host[2 * i].W + 31) / 32, (host[2 * i].H + 3) / 4);
             switch (prec) {
@@ -517,8 +521,11 @@ struct plbm_batch {
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
+        const unsigned long long before = issued;
         const cudaError_t el = enqueue_plain(0, steps_per_graph);
         e = cudaStreamEndCapture(stream, &g);
+        graph_kernels = issued - before;
+        issued = before;
         if (el != cudaSuccess) return el;
         if (e != cudaSuccess) return e;
         e = cudaGraphInstantiate(&gexec, g, 0);
@@ -677,6 +684,7 @@ int plbm_batch_run(plbm_batch *b, unsigned steps, int mode, double *ms_per_step)
         if (e == cudaSuccess) e = b->ensure_graph(per_graph);
         while (e == cudaSuccess && k + per_graph <= steps - 1) {
             e = cudaGraphLaunch(b->gexec, b->stream);
+            b->issued += b->graph_kernels;
             k += per_graph;
         }
     }
@@ -756,6 +764,13 @@ int plbm_batch_info(plbm_batch *b, unsigned long long *nodes, unsigned *tiles)
 {
     if (nodes) *nodes = b->nodes;
     if (tiles) *tiles = b->n_tiles;
+    return PLBM_OK;
+}
+
+int plbm_batch_launches(plbm_batch *b, unsigned long long *n)
+{
+    if (!n) return berr(b, PLBM_ERR_ARGUMENT, "n is NULL");
+    *n = b->issued;
     return PLBM_OK;
 }
 

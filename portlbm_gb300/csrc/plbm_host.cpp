@@ -457,6 +457,8 @@ struct plbm_handler {
     int outlet_mode = 0;
     // debugMode on nptl / lptl: the reference's unfused stream / observables / collide kernels
     bool debug = false;
+    std::atomic<unsigned long long> issued{ 0 };   // kernels of steps, graph replays counted by what they hold
+    unsigned long long graph_kernels = 0, frame_kernels[2] = { 0, 0 };
     int pair_rows = 0;     // rows a warp of the two-step kernel marches over; 0: one step a launch
     bool vec_rows = false, vec_results = false;   // nptl, 2-byte storage, stream layout: plain steps and steps
                                                   // with results by vectorised rows
@@ -877,6 +879,7 @@ struct plbm_handler {
         p.jy_prev = jy_d + (size_t)par * H;
         p.jy_next = jy_d + (size_t)(par ^ 1u) * H;
         if (alg == 2) { p.halo_in = (double *)halo[par]; p.halo_out = (double *)halo[par ^ 1u]; }
+        issued += debug ? 3 : 1;
         if (debug) return plbm::launch_debug_step(prec, lay, alg == 1, p, block, stream);
         switch (alg) {
         case 0: return plbm::launch_nptl(step_prec, lay, p, grid, block, stream, porous, results ? vec_results : vec_rows);
@@ -983,6 +986,7 @@ struct plbm_handler {
         p.lat1 = lat[par ^ 1u];
         p.jy_prev = jy_d + (size_t)par * H;
         p.jy_next = jy_d + (size_t)(par ^ 1u) * H;
+        ++issued;
         return plbm::launch_two_steps(prec, lay, p, pair_rows, stream);
     }
 
@@ -1006,8 +1010,11 @@ struct plbm_handler {
         const unsigned pairs = N >= (1ull << 22) ? 4 : 32;
         cudaGraph_t g = nullptr;
         cuda_check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
+        const unsigned long long before = issued;
         const cudaError_t e = enqueue_plain(0, 2 * pairs);
         cudaError_t e2 = cudaStreamEndCapture(stream, &g);
+        graph_kernels = issued - before;
+        issued = before;
         cuda_check(e, "capture launch");
         cuda_check(e2, "end capture");
         cuda_check(cudaGraphInstantiate(&gexec, g, 0), "graph instantiate");
@@ -1029,9 +1036,12 @@ struct plbm_handler {
         wait_host();   // the copies target the pinned host arrays
         cudaGraph_t g = nullptr;
         cuda_check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
+        const unsigned long long before = issued;
         cudaError_t e = enqueue_plain(t0, F - 1);
         if (e == cudaSuccess) e = launch_step(t0 + F - 1, true, true);
         cudaError_t e2 = cudaStreamEndCapture(stream, &g);
+        frame_kernels[par] = issued - before;
+        issued = before;
         cuda_check(e, "frame capture");
         cuda_check(e2, "end capture");
         cuda_check(cudaGraphInstantiate(&frame_gexec[par], g, 0), "graph instantiate");
@@ -1048,6 +1058,7 @@ struct plbm_handler {
             if (t & 1u) { cuda_check(launch_step(t, false), "step"); ++t; }
             while (t + graph_steps <= t1) {
                 cuda_check(cudaGraphLaunch(gexec, stream), "graph launch");
+                issued += graph_kernels;
                 t += graph_steps;
             }
         }
@@ -1140,6 +1151,7 @@ struct plbm_handler {
                 if (opt.use_graph && !export_fields && !debug && F >= 2 && F <= 256 && t % F == 0 && t + F < T) {
                     // a whole frame: one graph launch (its steps, results written to the host)
                     cuda_check(cudaGraphLaunch(frame_graph(t, F), stream), "frame graph launch");
+                    issued += frame_kernels[t & 1u];
                     host_results_newer = true;
                     end = t + F;
                 } else if (t < frame) {
@@ -1659,6 +1671,14 @@ int plbm_launches_per_step(plbm_handler *h, unsigned *n)
 {
     *n = h->debug ? 3 : 1;
     return PLBM_OK;
+}
+
+int plbm_launches(plbm_handler *h, unsigned long long *n)
+{
+    return guarded(h, [&] {
+        if (!n) fail(PLBM_ERR_ARGUMENT, "n is NULL");
+        *n = h->issued;
+    });
 }
 
 int plbm_run_launches(plbm_handler *h, unsigned n, unsigned *launches)
