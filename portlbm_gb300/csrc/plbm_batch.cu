@@ -335,6 +335,8 @@ struct plbm_batch {
     unsigned long long issued = 0, graph_kernels = 0;   // kernels of steps; those of a replay of gexec
     int pair_rows = 0;             // rows of a two-step launch's pieces; 0: single steps only (offsets too wide)
     unsigned pair_blocks = 0;
+    unsigned long long padded = 0, strip_rows = 0, warp_rows = 0;   // nodes with the rows' padding; rows times strips, and
+                                                                    // times a single step's warps
     unsigned *pair_domain_d = nullptr, *pair_first_d = nullptr;
     std::string err;
     unsigned long long nodes = 0;
@@ -440,10 +442,13 @@ struct plbm_batch {
     // 22 / 19 / 21; 6.9 M, 4 / 8 / 16: 78 / 75 / 79).
     cudaError_t build_pairs()
     {
-        unsigned long long padded = 0, offsets = 0;
+        unsigned long long offsets = 0;
         const size_t eb = prec == PLBM_F32 ? 4 : prec == PLBM_F64_Q60 ? 8 : 2;
         for (unsigned i = 0; i < n_domains(); ++i) {
-            padded += host[2 * i].N;
+            const StepParams &d = host[2 * i];
+            padded += d.N;
+            strip_rows += (unsigned long long)((d.W + plbm::PAIR_COLUMNS - 1) / plbm::PAIR_COLUMNS) * d.H;
+            warp_rows += (unsigned long long)(d.P / 32) * d.H;
             offsets = std::max<unsigned long long>(offsets, 9ull * host[2 * i].N * (eb == 8 ? 1 : eb));
         }
         if (offsets >= (1ull << 32)) return cudaSuccess;   // the kernel's offsets have 32 bits
@@ -464,6 +469,19 @@ struct plbm_batch {
         pair_blocks = (unsigned)dom.size();
         pair_rows = rows;
         return cudaSuccess;
+    }
+
+    // Whether they do: not where rows are so narrow that their strips of 30 columns are many more than warps of
+    // 32 nodes, against vectorised rows and for F64_Q60, whose single steps come closest.  us a step, single
+    // steps -> two a launch: 62 x h, three strips for two warps, f16s vectorised 1.0 M nodes 24 -> 23, 2.0 M
+    // 41.6 -> 45.2, 9.3 M 131 -> 160, 20 M 278 -> 349 (but plain tiles 427 -> 361), f64_q60 1.0 M 83 -> 57,
+    // 2.0 M 102 -> 107, 9.3 M 371 -> 407; 95 x h, four for three, f16s vectorised 9.1 M 131 -> 130, 20 M
+    // 273 -> 289, f64_q60 754 -> 750; 128 x h, five for four, f16s 20 M 267 -> 272, f16c 353 -> 348.
+    bool two_steps_pay() const
+    {
+        if (!vec() && prec != PLBM_F64_Q60) return true;
+        if (10 * strip_rows > 14 * warp_rows && padded >= (3ull << 19)) return false;
+        return !vec() || padded < (1ull << 24) || 10 * strip_rows <= 13 * warp_rows;
     }
 
     // Two steps in one launch from the lattices of parity `parity`, without results.
@@ -488,7 +506,7 @@ struct plbm_batch {
     cudaError_t enqueue_plain(unsigned t, unsigned n)
     {
         cudaError_t e = cudaSuccess;
-        for (; pair_rows && n >= 4 && e == cudaSuccess; t += 4, n -= 4) {
+        for (; pair_rows && n >= 4 && e == cudaSuccess && two_steps_pay(); t += 4, n -= 4) {
             e = launch_two_steps(t & 1u);
             if (e == cudaSuccess) e = launch_two_steps((t & 1u) ^ 1u);
         }

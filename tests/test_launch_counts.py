@@ -41,3 +41,27 @@ def test_batch(plbm):
     b.run(5, mode="per_domain")
     assert b.launches() == 17 + 15
     b.close()
+
+
+@pytest.mark.parametrize("precision,vec,w,h,copies,two", [
+    ("f16s", True, 62, 900, 20, True), ("f16s", True, 62, 1700, 20, False), ("f16s", False, 62, 1700, 20, True),
+    ("f16s", True, 95, 1700, 20, True), ("f16s", True, 95, 3000, 60, False), ("f16c", True, 128, 2300, 60, True),
+    ("f64_q60", False, 64, 1700, 20, False), ("f64_q60", False, 95, 1700, 20, True), ("f32", False, 62, 1700, 20, True)])
+def test_batches_of_narrow_domains(plbm, precision, vec, w, h, copies, two):
+    """Strips many more than warps: single steps where those are as good; the values are the same."""
+    m = (np.random.default_rng(w).random((h, w)) < 0.1).astype(np.int8)
+    doms = [{"mask": m, "relaxation_time": 0.7, "inlet_density": 1.02}] * copies
+    many, single = (plbm.Batch(doms, precision=precision) for _ in range(2))
+    for b in (many, single):
+        b.set_tile(32, 4 + 256 * 2 + (plbm.BATCH_TILE_VEC if vec else 0), 4)
+    many.run(9, mode="persistent")
+    assert many.launches() == (5 if two else 9)
+    many.run(18, mode="persistent_graph")
+    assert many.launches() == (5 + 10 if two else 27)    # an odd first step, 16 in 8 launches, one with results
+    for _ in range(27):
+        single.run(1)
+    for i in (0, copies - 1):
+        for which in range(3):
+            assert np.array_equal(many.result(i, which), single.result(i, which))
+    many.close()
+    single.close()
