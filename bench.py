@@ -454,7 +454,8 @@ def parse_batch_tile(text, plbm):
 
 def batch_study(plbm, steps=100, precisions=("f32", "f16s"), n=256, tile=None):
     """Aggregate MLUPS of `n` uneven domains: one persistent tile-queue launch per step replayed from a
-    CUDA graph (tiles autotuned, or `tile` = set_tile's arguments for the 2-byte forms) against one
+    CUDA graph (the tiles of the steps that go one by one autotuned, or `tile` = set_tile's arguments for the
+    2-byte forms) against one
     launch per domain per step."""
     doms = batch_domains(plbm, n=n)
     out = {"domains": len(doms)}

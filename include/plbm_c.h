@@ -295,8 +295,9 @@ void plbm_batch_destroy(plbm_batch *b);
  * 256 x ((tile_h & 255) * rows) nodes. */
 #define PLBM_BATCH_TILE_VEC 0x10000
 int plbm_batch_set_tile(plbm_batch *b, int tile_w, int tile_h, int blocks_per_sm);
-/* Times `steps` persistent steps for each candidate tile shape and occupancy, keeps the fastest
- * (the timed steps advance the batch). */
+/* Times `steps` single persistent steps for each candidate tile shape and occupancy, keeps the fastest
+ * (the timed steps advance the batch).  The tile shapes the steps that go one by one: those with results and
+ * left-over ones, and all of a batch that does not step two a launch. */
 int plbm_batch_autotune(plbm_batch *b, unsigned steps, int *tile_w, int *tile_h, int *blocks_per_sm);
 /* Advances every domain by `steps`; results are written on the last one.  Device ms per step. */
 int plbm_batch_run(plbm_batch *b, unsigned steps, int mode, double *ms_per_step);

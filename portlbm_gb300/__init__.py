@@ -536,6 +536,8 @@ class Batch:
         self._ok(self._lib.plbm_batch_set_tile(self._h, tile_w, tile_h, blocks_per_sm))
 
     def autotune(self, steps: int = 4) -> tuple:
+        """Times `steps` single steps of every candidate tile and keeps the fastest: the tile shapes the steps
+        that go one by one (with results, or left over), not two-step launches."""
         w, h, b = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         self._ok(self._lib.plbm_batch_autotune(self._h, steps, ctypes.byref(w), ctypes.byref(h), ctypes.byref(b)))
         return w.value, h.value, b.value

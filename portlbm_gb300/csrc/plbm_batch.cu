@@ -335,6 +335,7 @@ struct plbm_batch {
     unsigned long long issued = 0, graph_kernels = 0;   // kernels of steps; those of a replay of gexec
     int pair_rows = 0;             // rows of a two-step launch's pieces; 0: single steps only (offsets too wide)
     unsigned pair_blocks = 0;
+    bool tuning = false;           // plbm_batch_autotune runs: single steps only
     unsigned long long padded = 0, strip_rows = 0, warp_rows = 0;   // nodes with the rows' padding; rows times strips, and
                                                                     // times a single step's warps
     unsigned *pair_domain_d = nullptr, *pair_first_d = nullptr;
@@ -479,6 +480,7 @@ struct plbm_batch {
     // 273 -> 289, f64_q60 754 -> 750; 128 x h, five for four, f16s 20 M 267 -> 272, f16c 353 -> 348.
     bool two_steps_pay() const
     {
+        if (tuning) return false;
         if (!vec() && prec != PLBM_F64_Q60) return true;
         if (10 * strip_rows > 14 * warp_rows && padded >= (3ull << 19)) return false;
         return !vec() || padded < (1ull << 24) || 10 * strip_rows <= 13 * warp_rows;
@@ -749,7 +751,10 @@ int plbm_batch_autotune(plbm_batch *b, unsigned steps, int *tile_w, int *tile_h,
     auto tryit = [&](int w, int h, int k) {
         if (plbm_batch_set_tile(b, w, h, k) != PLBM_OK) return PLBM_OK;
         double ms = 0;
-        if (plbm_batch_run(b, steps, PLBM_BATCH_PERSISTENT, &ms) != PLBM_OK) return PLBM_ERR_CUDA;
+        b->tuning = true;   // the tile shapes single steps; a two-step launch does not depend on it
+        const int rc = plbm_batch_run(b, steps, PLBM_BATCH_PERSISTENT, &ms);
+        b->tuning = false;
+        if (rc != PLBM_OK) return PLBM_ERR_CUDA;
         if (ms < best) { best = ms; bw = w; bh = h; bb = k; }
         return PLBM_OK;
     };

@@ -65,3 +65,15 @@ def test_batches_of_narrow_domains(plbm, precision, vec, w, h, copies, two):
             assert np.array_equal(many.result(i, which), single.result(i, which))
     many.close()
     single.close()
+
+
+@pytest.mark.parametrize("precision,candidates", [("f32", 21), ("f16s", 42)])
+def test_autotune_times_single_steps(plbm, precision, candidates):
+    """The tile it chooses shapes steps with results and left-over ones, not two-step launches."""
+    doms = [{"mask": np.zeros((40, 50), np.int8), "relaxation_time": 0.7, "inlet_density": 1.02}]
+    b = plbm.Batch(doms, precision=precision)
+    b.autotune(9)
+    assert b.launches() == candidates * 9
+    b.run(9, mode="persistent")
+    assert b.launches() == candidates * 9 + 5
+    b.close()
