@@ -191,20 +191,6 @@ def forward_plan(n, h, w):
     return tuple(plan), at
 
 
-class Activations:
-    """The tensors of a forward pass by name ("in", "e0a", ..., "out"), made from its buffer when asked for."""
-
-    def __init__(self, x, work, plan, out):
-        self._work, self._plan = work, {name: (off, shape) for name, off, shape in plan}
-        self._given = {"in": x, "out": out}
-
-    def __getitem__(self, name):
-        if name in self._given:
-            return self._given[name]
-        off, shape = self._plan[name]
-        return self._work[off:off + math.prod(shape)].view(shape)
-
-
 class NeuralOperator:
     """U-Net-style operator; forward/backward/Adam all run in libplbm's kernels."""
 
@@ -227,6 +213,7 @@ class NeuralOperator:
         self.norm = np.array([1.0, 1.0])          # std of t_rho and of t_j over the training set
         self.step_count = 0
         self._s = None
+        self._acts = self._pieces = None
 
     def save(self, path):
         """Writes the FP32 master weights, biases and target scales to an .npz file."""
@@ -272,8 +259,24 @@ class NeuralOperator:
         layers = (_CLayer * len(self.layers))(*[_CLayer(l.wb.data_ptr(), l.b.data_ptr(), l.cin, l.cout, int(l.relu))
                                                 for l in self.layers])
         _ok(self.lib.plbm_nn_unet_forward(x.data_ptr(), acts, layers, LEVELS, n, h, w, self._s))
-        self.acts, self.shape = Activations(x, work, plan, out), (n, h, w)
+        self._acts, self._pieces, self.shape = None, (x, work, plan, out), (n, h, w)
         return out
+
+    @property
+    def acts(self):
+        """The tensors of the last forward pass by name ("in", "e0a", ..., "out"): views of its buffer, made when
+        first asked for."""
+        if self._acts is None:
+            if self._pieces is None:
+                raise AttributeError("acts: no forward pass has run")
+            x, work, plan, out = self._pieces
+            views = {name: work[off:off + math.prod(shape)].view(shape) for name, off, shape in plan}
+            self._acts = {"in": x, **views, "out": out}
+        return self._acts
+
+    @acts.setter
+    def acts(self, tensors):
+        self._acts = tensors
 
     def _relu_bwd(self, layer, y, n, h, w, g, source=GRAD, skip=None, out=None):
         """The gradient of a layer's convolution from that of its output, formed on the way from g
