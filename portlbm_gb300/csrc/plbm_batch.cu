@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(32 * PAIR_WARPS, PREC == F64_Q60 ? 5 : PREC ==
     __syncthreads();
     const int strips = (sp.W + PAIR_COLUMNS - 1) / PAIR_COLUMNS;
     const int ya = piece / strips * a.rows;
-    if (ya < sp.H) march_two_steps<PREC, STREAM, false>(sp, piece % strips, ya, min(ya + a.rows, sp.H));   // warp-uniform
+    if (ya < sp.H) march_two_steps<PREC, STREAM>(sp, piece % strips, ya, min(ya + a.rows, sp.H));   // warp-uniform
 }
 
 // One launch per domain with the same per-node update (the comparison the batching form is

@@ -299,8 +299,9 @@ __device__ __forceinline__ MomentsF collide_f32_ref(float f[9], float omega)
 }
 
 // The coefficients of collide_f32: from the step parameters, operands in constant memory; or formed for
-// the node from omega (the same products), for the batch kernels, whose parameters lie in shared memory
-// (k_batch_vec<F16S> on 20 domains 87.8 us a step, 93.4 with the coefficients read).
+// the node from omega (the same products), for the batch kernels that step singly, whose parameters lie in
+// shared memory (k_batch_vec<F16S> on 20 domains 87.8 us a step, 93.4 with the coefficients read).  The batch
+// kernel of two steps reads them from shared memory.
 struct CoefficientsF { float om1, ow49, ow9, ow36, k9, k36, o9, o36, r; };
 template <bool FORMED> __device__ __forceinline__ CoefficientsF coefficients(const StepParams &p, float qs)
 {
@@ -527,8 +528,8 @@ __device__ __forceinline__ void outlet_fill_float(float f[9], float hy, const St
 // Outlet populations 0, 3, 6 of a border node (X-2, y), y in [2, V-3], from its other pulled
 // values: OutletUpdateKernel non_buffered.hpp:95-129 with f_1 = f[1], f_4 = f[4], f_7 = f[7]
 // and f_inverse = {f[8], f[5], f[2]} (the same lattice entries).
-// BATCH: in a batch kernel, where half_jy's call costs more than it saves (k_batch_vec<F16S> 90.3 us a
-// step on 20 domains against 87.6).
+// BATCH: in a batch kernel of single steps, where half_jy's call costs more than it saves (k_batch_vec<F16S>
+// 90.3 us a step on 20 domains against 87.6).
 template <int PREC, bool BATCH = false>
 __device__ __forceinline__ void outlet_fill(typename Store<PREC>::C f[9], double jyo, const StepParams &p)
 {

@@ -44,14 +44,15 @@ template <int PREC> __device__ __forceinline__ CT<PREC> stored_value(CT<PREC> v,
     } else return v;
 }
 
-// Half of what the outlet of the next step reads of this step's jy in column W - 2 (write_observables'
-// jy_next), in the form's own scale: an exact product, as half_jy's.
-__device__ __forceinline__ double column_half_jy(const Moments &m, const StepParams &p)
+// What the outlet of the next step takes of this step's jy in column W - 2 (write_observables' jy_next):
+// for F64_Q60 the value itself, for the shifted forms half of it in the form's own scale, an exact product
+// as half_jy's.
+__device__ __forceinline__ double outlet_jy(const Moments &m, const StepParams &p)
 {
     const double v = q_to_double(__double_as_longlong(m.jy));
     return p.nan_protection ? nan_guard(v) : v;
 }
-__device__ __forceinline__ float column_half_jy(const MomentsF &m, const StepParams &p)
+__device__ __forceinline__ float outlet_jy(const MomentsF &m, const StepParams &p)
 {
     const bool drop = p.nan_protection && !(m.jy <= 3.40282347e38f);   // NaN or above FLT_MAX
     return drop ? 0.0f : 0.5f * m.jy;
@@ -137,9 +138,8 @@ __device__ __forceinline__ void pair_gather(CT<PREC> g[9], unsigned at, int xi, 
     if (lk & LINK_EDGE) fill_ghosts<PREC>(g, xi, yi, p);
 }
 
-// One warp's rows [ya, yb) of strip `strip` (at least one column of it in the domain).  BATCH: the
-// parameters lie in shared memory (see CoefficientsF).
-template <int PREC, int L, bool BATCH = false>
+// One warp's rows [ya, yb) of strip `strip` (at least one column of it in the domain).
+template <int PREC, int L>
 __device__ __forceinline__ void march_two_steps(const StepParams &p, int strip, int ya, int yb)
 {
     constexpr unsigned ALL = 0xffffffffu;
@@ -167,11 +167,11 @@ __device__ __forceinline__ void march_two_steps(const StepParams &p, int strip, 
         J jya = 0;
         if (lk & LINK_FLUID) {
             pair_gather<PREC, L>(a, at, xi, r, lk, p);
-            if (is_outlet_row(xi, r, p)) outlet_fill<PREC, BATCH>(a, jy_prev_at(p, r), p);
-            const auto m = collide<PREC, BATCH>(a, p);
+            if (is_outlet_row(xi, r, p)) outlet_fill<PREC>(a, jy_prev_at(p, r), p);
+            const auto m = collide<PREC>(a, p);
 #pragma unroll
             for (int d = 0; d < 9; ++d) a[d] = stored_value<PREC>(a[d], p);
-            if (PREC != F64_Q60 || xi == p.W - 2) jya = column_half_jy(m, p);
+            if (PREC != F64_Q60 || xi == p.W - 2) jya = outlet_jy(m, p);
         }
         // the second step's node (xi, r - 1): its sources are rows r - 2 (c), r - 1 (b) and r (a)
         const int y = r - 1;
@@ -205,7 +205,7 @@ __device__ __forceinline__ void march_two_steps(const StepParams &p, int strip, 
                         }
                     }
                 }
-                const auto m = collide<PREC, BATCH>(f, p);
+                const auto m = collide<PREC>(f, p);
 #pragma unroll
                 for (int d = 0; d < 9; ++d) {
                     using T = typename Store<PREC>::T;
