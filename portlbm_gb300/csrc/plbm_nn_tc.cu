@@ -156,27 +156,31 @@ struct TcArgs {
     int BW, BH, tiles_x, tiles_y;
     int stage_bytes;        // A tile + the B tile rounded up to 1024 B
     int stages;
-    int last_tap_first;     // accumulate the taps from the last to the first
+    int tap0, tap_step;     // order of the taps: tap0, tap0 + tap_step, ...
     int *err;
 };
 
-template <int KB>   // channels per K block: 32 or 64
+// KB: channels per K block, 32 or 64.  STAGES: a.stages where it is known at compile time, otherwise 0: layers
+// of 32-channel blocks with tiles for several CTAs an SM take four.  (With the ring's size and the order of the taps
+// worked out in the loop, 96 -> 128 channels of 40 x 256^2 pixels took 762 us instead of 745.)
+template <int KB, int STAGES>
 __global__ void __launch_bounds__(128, 4)
 k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, TcArgs a)
 {
+    const int nstages = STAGES ? STAGES : a.stages;
     __shared__ float s_bias[128];
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
     // stages aligned to 1024 B (the swizzle pattern repeats every 512 B)
     unsigned char *smem = tc_smem_raw + ((1024 - (smem_u32(tc_smem_raw) & 1023)) & 1023);
-    unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem + a.stages * a.stage_bytes);
-    unsigned long long *full = bars, *empty = bars + a.stages, *done = bars + 2 * a.stages;
-    unsigned *tmem_slot = reinterpret_cast<unsigned *>(bars + 2 * a.stages + 1);
+    unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem + nstages * a.stage_bytes);
+    unsigned long long *full = bars, *empty = bars + nstages, *done = bars + 2 * nstages;
+    unsigned *tmem_slot = reinterpret_cast<unsigned *>(bars + 2 * nstages + 1);
     int *counts = reinterpret_cast<int *>(tmem_slot + 1);   // [0] issued, [1] consumed, [2] failed
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned ncols = a.npad <= 32 ? 32u : (a.npad <= 64 ? 64u : 128u);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < a.stages; ++s) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
+        for (int s = 0; s < nstages; ++s) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
         mbar_init(smem_u32(done), 1);
         counts[0] = counts[1] = counts[2] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -207,12 +211,12 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
     const unsigned abytes = TC_BM * KB * 2, bbytes = (unsigned)a.npad * KB * 2;
 
     if (warp == 0 && lane == 0) {              // producer: TMA loads
-        for (int it = 0, s = 0, round = 0; it < iters; ++it, s = s + 1 == a.stages ? (++round, 0) : s + 1) {
+        for (int it = 0, s = 0, round = 0; it < iters; ++it, s = s + 1 == nstages ? (++round, 0) : s + 1) {
             if (round > 0 && !mbar_wait(smem_u32(&empty[s]), (unsigned)((round - 1) & 1))) {
                 counts[2] = 1;
                 break;
             }
-            const int kb = it % kblocks, tap = a.last_tap_first ? 8 - it / kblocks : it / kblocks;
+            const int kb = it % kblocks, tap = a.tap0 + a.tap_step * (it / kblocks);
             const int dy = tap / 3 - 1, dx = tap % 3 - 1;
             unsigned char *st = smem + s * a.stage_bytes;
             const unsigned bar = smem_u32(&full[s]);
@@ -223,7 +227,7 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
         }
     } else if (warp == 1 && lane == 0) {       // MMA issuer
         const unsigned idesc = instr_desc(a.npad);
-        for (int it = 0, s = 0, round = 0; it < iters; ++it, s = s + 1 == a.stages ? (++round, 0) : s + 1) {
+        for (int it = 0, s = 0, round = 0; it < iters; ++it, s = s + 1 == nstages ? (++round, 0) : s + 1) {
             if (!mbar_wait(smem_u32(&full[s]), (unsigned)(round & 1))) {
                 counts[2] = 1;
                 break;
@@ -265,7 +269,7 @@ k_conv_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
         // flight (their stages' full barriers), each bounded, before the TMEM is released
         mbar_wait(smem_u32(done), 0);
         for (int it = counts[1]; it < counts[0]; ++it)
-            mbar_wait(smem_u32(&full[it % a.stages]), (unsigned)((it / a.stages) & 1));
+            mbar_wait(smem_u32(&full[it % nstages]), (unsigned)((it / nstages) & 1));
     }
     __syncthreads();
     if (warp == 0) {
@@ -1317,9 +1321,9 @@ int plbm_nn_tc_conv(const void *x, const void *w, const float *bias, void *y, in
     {
         std::lock_guard<std::mutex> g(mu);
         if (!attr) {
-            if (cudaFuncSetAttribute(k_conv_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess ||
-                cudaFuncSetAttribute(k_conv_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess)
-                return PLBM_ERR_CUDA;
+            for (auto kernel : { k_conv_tc<32, 0>, k_conv_tc<32, TC_STAGES>, k_conv_tc<64, 0> })
+                if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess)
+                    return PLBM_ERR_CUDA;
             attr = true;
         }
     }
@@ -1397,9 +1401,11 @@ int plbm_nn_tc_conv(const void *x, const void *w, const float *bias, void *y, in
     const int fit = (TC_SMEM - 1024 - 256) / stage, most = fit < TC_MAX_STAGES ? fit : TC_MAX_STAGES;
     const int stages = ctas <= sms ? most : ctas <= 2 * sms ? (most + 1) / 2 : TC_STAGES * TC_KB / kb;
     if (!maps(kb, npart)) return PLBM_ERR_ARGUMENT;
+    const bool last_first = dgrad && !tiles_exactly(H, W);
     TcArgs a{ (__nv_bfloat16 *)y, bias, N, H, W, Cin, Cout, npart, relu, BW, BH, t.x, t.y, stage, stages,
-              dgrad && !tiles_exactly(H, W), err };
-    return nn_launch(kb == 64 ? k_conv_tc<64> : k_conv_tc<32>, dim3((unsigned)tiles, (unsigned)parts), 128,
+              last_first ? 8 : 0, last_first ? -1 : 1, err };
+    const auto kernel = kb == 64 ? k_conv_tc<64, 0> : stages == TC_STAGES ? k_conv_tc<32, TC_STAGES> : k_conv_tc<32, 0>;
+    return nn_launch(kernel, dim3((unsigned)tiles, (unsigned)parts), 128,
                      (size_t)stages * stage + 1024 + 256, s, xmap, wmap, a) == cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
 }
 
