@@ -379,8 +379,8 @@ int plbm_nn_adam_dev(float *w, const float *g, float *m, float *v, void *w_bf16,
  * exchanged.  Other shapes, and buffers that do not start on 16 bytes, run the mma.sync kernel. */
 int plbm_nn_conv_on_tensor_cores(int H, int W, int Cin, int Cout);
 /* 1 when plbm_nn_conv_wgrad runs the shape on tcgen05: Cout <= 128, and either Cin a multiple of 32 up
- * to 128 (TMA-fed input tiles) or Cin <= 32 on the images above (im2col tiles written by the CTA's
- * threads). */
+ * to 128 (TMA-fed input tiles; a batch of at most 1400 pixels that the tiles do not cover exactly may
+ * still run mma.sync) or Cin <= 32 on the images above (im2col tiles written by the CTA's threads). */
 int plbm_nn_wgrad_on_tensor_cores(int H, int W, int Cin, int Cout);
 /* Synchronises the device and reports whether a tensor-core convolution gave up on a wait (its
  * output is then invalid); clears the flag. */

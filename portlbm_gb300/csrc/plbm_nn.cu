@@ -20,6 +20,7 @@ int plbm_nn_tc_conv(const void *x, const void *w, const float *bias, void *y, in
                     int relu, bool dgrad, cudaStream_t s);
 int plbm_nn_tc_flip(const void *w, void *wt, int Cin, int Cout, cudaStream_t s);
 bool plbm_nn_tc_wgrad_supported(int H, int W, int Cin, int Cout);
+bool plbm_nn_tc_wgrad_pays(int N, int H, int W, int Cin, int Cout, bool bias);
 int plbm_nn_tc_wgrad(const void *x, const void *g, float *gw, float *gb, int N, int H, int W, int Cin, int Cout,
                      int *bias_done, cudaStream_t s);
 bool plbm_nn_tc_small_supported(int H, int W, int Cin, int Cout);
@@ -745,7 +746,7 @@ int plbm_nn_conv_wgrad(const void *x, const void *g, float *gw, float *gb, int N
 {
     int rc;
     const bool aligned = aligned16(x, g, nullptr);
-    if (aligned && plbm_nn_tc_wgrad_supported(H, W, Cin, Cout)) {
+    if (aligned && plbm_nn_tc_wgrad_supported(H, W, Cin, Cout) && plbm_nn_tc_wgrad_pays(N, H, W, Cin, Cout, gb != nullptr)) {
         int bias_done = 0;
         rc = plbm_nn_tc_wgrad(x, g, gw, gb, N, H, W, Cin, Cout, &bias_done, (cudaStream_t)stream);
         if (bias_done) gb = nullptr;   // the bias gradient came with the weight gradient

@@ -1417,6 +1417,17 @@ bool plbm_nn_tc_wgrad_supported(int H, int W, int Cin, int Cout)
     return H >= 1 && W >= 1 && Cin % TC_KB == 0 && Cin >= TC_KB && Cin <= 128 && Cout >= 1 && Cout <= WG_M;
 }
 
+// Whether it pays: not for a few hundred pixels of images that 128-pixel tiles cover badly, which a CTA's set-up and
+// its atomic additions then bound.  us with mma.sync / here, 4 x 4 and 8 x 8 images, 256 pixels: 64 -> 64 channels
+// 8.5 / 10.5, 96 -> 96 10.4 / 14.6, 128 -> 128 12.5 / 20.6; 640 pixels: 96 -> 64 10.6 / 12.7, but 128 -> 128 25.7 / 20.6;
+// 1024 pixels: 32 -> 128 13.6 / 18.7, 64 -> 64 14.5 / 10.4.  With the bias gradient, a kernel of its own beside
+// mma.sync's, only where many channels make the difference (256 pixels, 64 -> 64: 12.4 / 10.4, 96 -> 96 13.5 / 15.4).
+bool plbm_nn_tc_wgrad_pays(int N, int H, int W, int Cin, int Cout, bool bias)
+{
+    const long long few = Cin == 32 ? 1400 : Cin <= 96 ? 640 : 512;
+    return tiles_exactly(H, W) || (long long)N * H * W > few || (bias && Cin * Cout < 96 * 96 && Cout <= 96);
+}
+
 // gw[co][tap][ci] += sum_p g[p][co] x[p + tap][ci] on the tensor cores (x, g NHWC BF16, gw FP32); with
 // gb, also gb[co] += sum_p g[p][co] where a tile of ones fits the stage without another M tile
 // (*bias_done = 1; the caller then runs no bias kernel).
