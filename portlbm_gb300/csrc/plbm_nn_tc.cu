@@ -337,9 +337,11 @@ __device__ __forceinline__ int ws_mstart(int mt, int chunks) { return chunks > 4
 // aligned: the unit index is XORed with bits 7..8 of the unswizzled offset, i.e. (r / 2) mod 4.
 __device__ __forceinline__ unsigned sw64_off(int r, int u) { return (unsigned)(r * 64 + ((u ^ ((r >> 1) & 3)) << 4)); }
 
+// The loads of the kernels that are launched dependently are plain ones: a read-only load (__ldg) promises data that
+// does not change while the kernel is there, which the kernel before it may still be writing.
 __device__ __forceinline__ unsigned short ld_bf16_bits(const __nv_bfloat16 *p)
 {
-    return __ldg(reinterpret_cast<const unsigned short *>(p));
+    return *reinterpret_cast<const unsigned short *>(p);
 }
 
 // Unit U (channels 8U .. 8U + 7, zero past C) of pixel (n, py, px) of an NHWC tensor.
@@ -727,7 +729,7 @@ __device__ __forceinline__ uint4 im2col_unit(const __nv_bfloat16 *src, int C, in
         const int tap = c0 / C, ch = c0 - tap * C;
         const int sy = py + tap / 3 - 1, sx = px + tap % 3 - 1;
         if (tap < 9 && sy >= 0 && sy < H && sx >= 0 && sx < W)
-            return __ldg(reinterpret_cast<const uint4 *>(src + (((size_t)n * H + sy) * W + sx) * C + ch));
+            return *reinterpret_cast<const uint4 *>(src + (((size_t)n * H + sy) * W + sx) * C + ch);
         return make_uint4(0u, 0u, 0u, 0u);
     }
     if (C == 4) {       // two taps of four channels: two 8-byte loads
@@ -736,7 +738,7 @@ __device__ __forceinline__ uint4 im2col_unit(const __nv_bfloat16 *src, int C, in
             const int tap = 2 * U + h;
             const int sy = py + tap / 3 - 1, sx = px + tap % 3 - 1;
             if (tap < 9 && sy >= 0 && sy < H && sx >= 0 && sx < W) {
-                const uint2 q = __ldg(reinterpret_cast<const uint2 *>(src + (((size_t)n * H + sy) * W + sx) * 4));
+                const uint2 q = *reinterpret_cast<const uint2 *>(src + (((size_t)n * H + sy) * W + sx) * 4);
                 v[2 * h] = q.x;
                 v[2 * h + 1] = q.y;
             }
@@ -769,7 +771,7 @@ __device__ __forceinline__ void im2col_row(const __nv_bfloat16 *src, int H, int 
         if ((dy >= 0 || above) && (dy <= 0 || below) && (dx >= 0 || left) && (dx <= 0 || right)) {
             const __nv_bfloat16 *p = centre + ((long long)dy * W + dx) * C;
             if constexpr (C == 4) {
-                const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p));
+                const uint2 q = *reinterpret_cast<const uint2 *>(p);
                 v[2 * tap] = q.x;
                 v[2 * tap + 1] = q.y;
             } else {
