@@ -755,14 +755,14 @@ __device__ __forceinline__ uint4 im2col_unit(const __nv_bfloat16 *src, int C, in
     return make_uint4(v[0], v[1], v[2], v[3]);
 }
 
-// The im2col row of pixel (n, py, px) for C = 3 or 4 channels (the fields and the input of the operator), its
-// 9 C columns as CHUNKS * 16 words of two: the taps are compile-time, so no unit computes where its columns lie.
-template <int C, int CHUNKS>
+// The im2col row of pixel (n, py, px) of C channels, its 9 C columns as WORDS words of two: the taps are
+// compile-time, so no unit computes where its columns lie.
+template <int C, int WORDS>
 __device__ __forceinline__ void im2col_row(const __nv_bfloat16 *src, int H, int W, int n, int py, int px,
-                                           uint32_t (&v)[CHUNKS * 16])
+                                           uint32_t (&v)[WORDS])
 {
 #pragma unroll
-    for (int i = 0; i < CHUNKS * 16; ++i) v[i] = 0u;
+    for (int i = 0; i < WORDS; ++i) v[i] = 0u;
     const bool above = py > 0, below = py + 1 < H, left = px > 0, right = px + 1 < W;
     const __nv_bfloat16 *centre = src + (((size_t)n * H + py) * W + px) * C;
 #pragma unroll
@@ -774,6 +774,9 @@ __device__ __forceinline__ void im2col_row(const __nv_bfloat16 *src, int H, int 
                 const uint2 q = *reinterpret_cast<const uint2 *>(p);
                 v[2 * tap] = q.x;
                 v[2 * tap + 1] = q.y;
+            } else if constexpr (C % 2 == 0) {
+#pragma unroll
+                for (int k = 0; k < C / 2; ++k) v[tap * (C / 2) + k] = reinterpret_cast<const uint32_t *>(p)[k];
             } else {
 #pragma unroll
                 for (int ch = 0; ch < C; ++ch) {
@@ -806,7 +809,9 @@ struct SmallArgs {
 // latencies (loads, MMAs, accumulator, stores), so several CTAs share an SM, each walks every gridDim.x-th
 // tile, and the next tile's rows are written to a second buffer while the MMAs of this one run.
 // (A CTA of its own for every tile, with its set-up and weights: 16 x 256^2, 4 -> 32 channels, 54 -> 45 us;
-// the head's input gradient, 3 -> 32, 89 -> 36 us; with the taps of im2col_row computed per unit 60 and 94.)
+// the head's input gradient, 3 -> 32, 89 -> 36 us; with the taps computed per 16-byte unit of a row 60 and 94, and
+// 7 -> 16 channels 152 -> 159.)
+template <int CIN>   // 1 to 7
 __global__ void __launch_bounds__(SM_BUILD, 6) k_conv_small_tc(SmallArgs a)
 {
     __shared__ float s_bias[128];
@@ -840,33 +845,17 @@ __global__ void __launch_bounds__(SM_BUILD, 6) k_conv_small_tc(SmallArgs a)
     auto build = [&](int tile, unsigned char *to) {   // A: the thread writes its pixel's row
         int n, py, px;
         origin(tile, n, py, px);
-        auto store = [&](const auto &v) {
+        constexpr int WORDS = (9 * CIN + TC_KB - 1) / TC_KB * (TC_KB / 2);
+        uint32_t v[WORDS];
+        im2col_row<CIN>(a.x, a.H, a.W, n, py, px, v);
 #pragma unroll
-            for (int k = 0; k < (int)(sizeof(v) / 16); ++k)
-                *reinterpret_cast<uint4 *>(to + (k >> 2) * WG_CHUNK + sw64_off(row, k & 3)) =
-                    make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-        };
-        if (a.Cin == 4) {
-            uint32_t v[32];
-            im2col_row<4, 2>(a.x, a.H, a.W, n, py, px, v);
-            return store(v);
-        }
-        if (a.Cin == 3) {
-            uint32_t v[16];
-            im2col_row<3, 1>(a.x, a.H, a.W, n, py, px, v);
-            return store(v);
-        }
-        for (int c = 0; c < a.kchunks; ++c) {
-            uint4 u[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) u[k] = im2col_unit(a.x, a.Cin, a.H, a.W, n, py, px, c * 4 + k);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4 *>(to + c * WG_CHUNK + sw64_off(row, k)) = u[k];
-        }
+        for (int k = 0; k < WORDS / 4; ++k)
+            *reinterpret_cast<uint4 *>(to + (k >> 2) * WG_CHUNK + sw64_off(row, k & 3)) =
+                make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     };
     int tile = blockIdx.x;
     build(tile, As);
-    const int K = 9 * a.Cin;
+    constexpr int K = 9 * CIN;
     for (int i = threadIdx.x; i < a.kchunks * a.npad * 4; i += SM_BUILD) {   // B: row j = output channel j
         const int c = i / (a.npad * 4), rem = i - c * a.npad * 4, j = rem >> 2, k = rem & 3;
         uint32_t v[4] = { 0u, 0u, 0u, 0u };
@@ -1567,12 +1556,16 @@ int plbm_nn_tc_small_conv(const void *x, const void *w, const float *bias, void 
     a.BW = W >= TC_BM ? TC_BM : W; a.BH = TC_BM / a.BW; a.tiles_x = W / a.BW; a.tiles_y = H / a.BH;
     a.kchunks = (9 * Cin + TC_KB - 1) / TC_KB;
     a.err = err;
-    const int smem = a.kchunks * (2 * WG_CHUNK + a.npad * 64) + 1024 + 64;   // at most 42 KB
+    // at most 42 KB; at least so much that a seventh block finds no room on an SM, where dependent launches would put
+    // it while others have five (16 x 256^2, 3 -> 32 channels: 36.5 us, 31.9 with six on each)
+    const int need = a.kchunks * (2 * WG_CHUNK + a.npad * 64) + 1024 + 64, smem = need < 33 * 1024 ? 33 * 1024 : need;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
     a.total_tiles = N * a.tiles_x * a.tiles_y;
     const int ctas = sms * 6;   // six share an SM (38 KB each at 4 -> 32 channels); fewer tiles: one each
-    return nn_launch(k_conv_small_tc, (unsigned)(a.total_tiles < ctas ? a.total_tiles : ctas), SM_BUILD, smem, s, a) ==
+    static void (*const kernels[])(SmallArgs) = { k_conv_small_tc<1>, k_conv_small_tc<2>, k_conv_small_tc<3>, k_conv_small_tc<4>,
+                                                  k_conv_small_tc<5>, k_conv_small_tc<6>, k_conv_small_tc<7> };
+    return nn_launch(kernels[Cin - 1], (unsigned)(a.total_tiles < ctas ? a.total_tiles : ctas), SM_BUILD, smem, s, a) ==
                    cudaSuccess ? PLBM_OK : PLBM_ERR_CUDA;
 }
 
