@@ -74,9 +74,9 @@ __device__ __forceinline__ void emit_observables(const MomentsOf<PREC> &m, int x
 
 // Launch bounds of the nptl, lptl and npol step kernels: the Q60 form runs 256-thread blocks and
 // is limited by memory latency, so it is held to 48 registers for a fifth resident block per SM
-// (measured faster despite a few spilled words; nsol measured equal and keeps its registers).
-// F64_STRICT takes 80 registers for three blocks: 4096 x 4096 16.2 k MLUPS against 14.7 k with two
-// (105 registers) and 15.8 k with four (64, spills).
+// (measured faster despite a few spilled words; nsol's kernels are bounded by NsolBlocks).
+// F64_STRICT takes 80 registers for three blocks: 10 % faster than two (105 registers) and 3 % faster than
+// four (64, spills) when it was chosen; 4096 x 4096 17.7 k MLUPS now.
 template <int PREC> struct NptlBounds { static constexpr int threads = 512, blocks = 1; };
 template <> struct NptlBounds<F64_Q60> { static constexpr int threads = 256, blocks = 5; };
 template <> struct NptlBounds<F64_STRICT> { static constexpr int threads = 256, blocks = 3; };
@@ -842,8 +842,8 @@ __device__ __forceinline__ void nsol_odd_gather(CT<PREC> f[9], unsigned long lon
     }
 }
 
-// Q60: five blocks (48 registers): 8192 x 8192 stream 44.2 k MLUPS, 41.0 k without a bound; three, four
-// and six blocks measured 15, 6 and 2 % slower.  F64_PLAIN: 2000 x 500 stream 192 us a step, 202 without one.
+// Q60: five blocks (48 registers): 8192 x 8192 stream 41.2 k MLUPS, 38.7 k without a bound, bundle 42.4 k and
+// 39.4 k (in L2, 2000 x 500, 24.0 us a step and 23.2); three, four and six blocks measured 15, 6 and 2 % slower.  F64_PLAIN: 2000 x 500 stream 192 us a step, 202 without one.
 template <int PREC> struct NsolBlocks { static constexpr int value = PREC == F64_Q60 ? 5 : 3; };
 template <int PREC, int L> __global__ void k_nsol_even(StepParams p) { nsol_even_step<PREC, L>(p); }
 template <int PREC, int L> __global__ void __launch_bounds__(256, NsolBlocks<PREC>::value) k_nsol_even_bound(StepParams p)

@@ -8,7 +8,7 @@
 // kernel before it in the stream: everything that reads or writes activations or parameters comes
 // after nn_begin, which waits for that kernel and lets the next one in.  Tensor memory is allocated
 // before nn_begin, so the next kernel's blocks never hold columns that this kernel still waits for.
-// (A 1 x 256^2 inference of 39 launches: 226 -> 215 us as a graph.)
+// (A 1 x 256^2 inference of 31 launches: 226 -> 215 us as a graph.)
 __device__ __forceinline__ void nn_begin()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -67,15 +67,15 @@ PLBM_HD long long mulv(long long a, long long b)
 // below 1 for relaxation_time > 0.5 and is applied with mulc; omega f uses omega/2 twice.  The ALU
 // pipe bounds the kernels beside HBM: without the sign corrections that positive factors never need,
 // and with the range tested on high words, a node takes 484 instead of 522 instructions (k_nptl,
-// 4096 x 4096: ALU pipe 61 -> 45 % busy), the same values.  8192 x 8192 nptl stream 44.9 k -> 47.7 k
-// MLUPS, 2000 x 500 34.5 k -> 38.9 k, 1024 x 256 30.3 k -> 36.0 k.  (Weights factored into powers
+// 4096 x 4096: ALU pipe 61 -> 45 % busy), the same values.  One step a launch, nptl stream: 8192 x 8192 1607 ->
+// 1528 us, 2000 x 500 29.2 -> 26.3, 1024 x 256 8.6 -> 7.3 (with the dependent launches).  (Weights factored into powers
 // of two times 1/9 need 12 constant products and reach 50.1 k, but round differently: |j| near rest,
 // the square root of a few units of 2^-60, then moves by more than 1e-9.)
 // POSITIVE: no population and no R below zero, nearly every node of a flow; 12 of the 20 constant
 // products then need no correction for a negative factor.
 template <bool POSITIVE>
-PLBM_HD void relax_q60(long long f[9], long long jx, long long jy, long long jx2, long long jy2,
-                                          long long jxy, long long R, const StepParams &p)
+PLBM_HD void relax_q60(long long f[9], long long jx, long long jy, long long jx2, long long jy2, long long jxy,
+                       long long R, const StepParams &p)
 {
     const unsigned long long wh = (unsigned long long)p.q_om1;   // omega / 2, Q64
     const long long usq = jx2 + jy2;

@@ -8,7 +8,7 @@
 // rounded once to nearest, ties to even.  What stays on the FP64 pipe (25 operations) are the
 // products of two variables and the last relaxation step, whose operands have no common scale.
 //
-// Measured (k_nptl<F64_STRICT, STREAM>, 4096 x 4096): 5.7 k -> 17.8 k MLUPS; 2000 x 500: npol records
+// Measured (k_nptl<F64_STRICT, STREAM>, 4096 x 4096): 5.7 k -> 17.7 k MLUPS; 2000 x 500: npol records
 // 194 -> 72.4 us a step, nsol stream 194 -> 62.1 us.  With 25 FP64 instructions and about 780 on the ALU pipe
 // a warp both pipes are 70 % busy (the plain sequence keeps the FP64 pipe full); each further
 // operation moved off the FP64 pipe costs 12 to 30 ALU instructions against its 32 ALU slots' time.

@@ -247,7 +247,7 @@ class NeuralOperator:
         """x: [n,h,w,4] bf16 input; returns the [n,h,w,3] prediction and keeps activations for backward.
         h and w are multiples of 16 (four halvings); other extents raise RuntimeError.
 
-        One native call launches every kernel (39 launches from Python took longer than they ran); the
+        One native call launches every kernel (31 launches from Python took longer than they ran); the
         activations are pieces of one buffer, the prediction a tensor of its own."""
         self._s = self._stream()
         torch = self.torch
